@@ -92,6 +92,17 @@ __device__ __forceinline__ float blk_unscale(uint32_t max_bits) {
 }
 constexpr float kBlkLoScale = 2048.f;  // of the lo halves
 
+// v, a sum of products of scaled operands, with both scalings taken out, the smaller factor first: v is at
+// least about 1, so that neither step leaves the range of fp32 unless the result does.
+__device__ __forceinline__ float blk_unscaled(float v, uint32_t row_max, uint32_t col_max) {
+    const float a = blk_unscale(row_max), b = blk_unscale(col_max);
+    return v * fminf(a, b) * fmaxf(a, b);
+}
+__device__ __forceinline__ float4 blk_unscaled4(const float4& v, uint32_t row_max, const uint4& m) {
+    return make_float4(blk_unscaled(v.x, row_max, m.x), blk_unscaled(v.y, row_max, m.y), blk_unscaled(v.z, row_max, m.z),
+                       blk_unscaled(v.w, row_max, m.w));
+}
+
 // Two values times s as fp16 pairs: hi, and lo (s2 = s * 2^11).
 __device__ __forceinline__ void blk_split2(float x, float y, float s, float s2, uint32_t& hi, uint32_t& lo) {
     const __half2 h = __floats2half2_rn(x * s, y * s);
@@ -247,8 +258,8 @@ k_block_tc(const __half* __restrict__ X, int64_t m_tiles, int64_t k_chunks, cons
                 const int64_t row = cur.tile * 128 + xrow;
                 const int col0 = cur.panel * r + ch * 64;
                 const bool store = !direct || row < rows;
-                float u = 1.f;
-                if (direct && store) u = blk_unscale(__ldg(row_max + row));
+                uint32_t row_word = 0u;
+                if (direct && store) row_word = __ldg(row_max + row);
                 float* dst = direct ? direct + row * ldc + col0
                                     : partial + (((cur.split * panels + cur.panel) * m_tiles + cur.tile) * 128 + xrow) * (int64_t)r + ch * 64;
 #pragma unroll
@@ -264,8 +275,7 @@ k_block_tc(const __half* __restrict__ X, int64_t m_tiles, int64_t k_chunks, cons
                             float4 x = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
                             if (direct) {
                                 const uint4 m = __ldg((const uint4*)(col_max + col0 + g * 16 + j));
-                                x = make_float4(x.x * u * blk_unscale(m.x), x.y * u * blk_unscale(m.y),
-                                                x.z * u * blk_unscale(m.z), x.w * u * blk_unscale(m.w));
+                                x = blk_unscaled4(x, row_word, m);
                             }
                             if (store) *(float4*)(dst + g * 16 + j) = x;
                         }
@@ -475,10 +485,7 @@ __global__ void k_block_reduce(const float* __restrict__ partial, int n_split, i
         float4 b = p[(int64_t)s * rows_pad * r4];
         a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
     }
-    const float u = blk_unscale(__ldg(row_max + i));
-    const uint4 m = __ldg((const uint4*)col_max + c);
-    out[idx] = make_float4(a.x * u * blk_unscale(m.x), a.y * u * blk_unscale(m.y), a.z * u * blk_unscale(m.z),
-                           a.w * u * blk_unscale(m.w));
+    out[idx] = blk_unscaled4(a, __ldg(row_max + i), __ldg((const uint4*)col_max + c));
 }
 
 // Ranks up to 128 in one panel; 256, 384 and 512 as panels of 128 columns of Y and C.

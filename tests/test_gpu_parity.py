@@ -335,6 +335,26 @@ def test_op_block_product_scales(torch_cuda, M, K, r):
     assert np.all(np.abs(got - want) <= 2e-6 * want)
 
 
+@pytest.mark.parametrize("M,K,r", [(5, 40, 32), (300, 2000, 256)])
+@pytest.mark.parametrize("x_size,y_size", [(1e34, 1e-20), (1e-30, 1e30), (1e36, 1e-2)])
+def test_op_block_product_opposite_scales(torch_cuda, M, K, r, x_size, y_size):
+    """A huge X against a tiny Y and the reverse: what the operands were scaled by leaves the sum without
+    an intermediate that overflows (1e34 * 1e-20 is far inside fp32; with the scaling of X alone taken out the
+    sum is beyond 2^128)."""
+    from npeff_ref_b200._lib import lib, check
+    torch = torch_cuda
+    rng = np.random.default_rng(M + r)
+    X = (rng.uniform(0.5, 1.0, (M, K)) * x_size).astype(np.float32)
+    Y = (rng.uniform(0.5, 1.0, (K, r)) * y_size).astype(np.float32)
+    want = X.astype(np.float64) @ Y.astype(np.float64)
+    dX, dY = _dev(torch, X), _dev(torch, Y)
+    C_ = torch.full((M, r), float("nan"), device="cuda")
+    check(lib().dnpeff_op_block_product(dX.data_ptr(), M, K, dY.data_ptr(), r, C_.data_ptr(),
+                                        torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    assert np.all(np.abs(C_.cpu().numpy() - want) <= 2e-6 * want)
+
+
 # ---------------------------------------------------------------------------
 CASES = [
     # n, m, k, r, iters, eps
