@@ -112,6 +112,9 @@ struct dnpeff_engine {
     uint32_t* x1_max = nullptr;  // bits of the largest magnitude per row of x1; then
     uint32_t* x2_max = nullptr;  // per row of x2, and
     uint32_t* y_max[2] = {nullptr, nullptr};  // per column of the factor, of products in turn (ld words each)
+    unsigned long long* x1_sum = nullptr;     // sums that say where the halves do not do (blk_faint), per row of x1; then
+    unsigned long long* x2_sum = nullptr;     // per row of x2, and
+    unsigned char* blk_again = nullptr;       // a byte per row of a product
     __half* blk_ysplit = nullptr;
     float* blk_partial = nullptr;
 
@@ -350,7 +353,7 @@ void free_matrix(dnpeff_engine* e) {
     dev_free(e, e->new_to_og);
     dev_free(e, e->perm); dev_free(e, e->inv_perm);
     dev_free(e, e->b_vals); dev_free(e, e->b_col); dev_free(e, e->tail_off);
-    dev_free(e, e->x1); dev_free(e, e->x2); dev_free(e, e->x1_max); dev_free(e, e->blk_ysplit); dev_free(e, e->blk_partial);
+    dev_free(e, e->x1); dev_free(e, e->x2); dev_free(e, e->x1_max); dev_free(e, e->x1_sum); dev_free(e, e->blk_ysplit); dev_free(e, e->blk_partial);
     e->tail_nnz.clear();
     e->n_hot = 0; e->n_tail_blocks = 0; e->hot_nnz = 0;
     dev_free(e, e->W); dev_free(e, e->H); dev_free(e, e->AHG); dev_free(e, e->WA); dev_free(e, e->WW);
@@ -789,6 +792,11 @@ int load_device(dnpeff_engine* e, int64_t n, int64_t m_full, int64_t k, const in
             e->y_max[0] = e->x2_max + e->plan_x2.xmax_words;
             e->y_max[1] = e->y_max[0] + ld;
             DN_CUDA(cudaMemsetAsync(e->x1_max, 0, sizeof(uint32_t) * maxima, st));
+            const size_t sums = e->plan_x1.xmax_words + e->plan_x2.xmax_words, flags8 = (size_t)(std::max(n, n_hot) + 7) / 8;
+            DN_TRY(dev_alloc(e, &e->x1_sum, sums + flags8));
+            e->x2_sum = e->x1_sum + e->plan_x1.xmax_words;
+            e->blk_again = (unsigned char*)(e->x1_sum + sums);
+            DN_CUDA(cudaMemsetAsync(e->x1_sum, 0, sizeof(*e->x1_sum) * (sums + flags8), st));
             DN_TRY(dev_alloc(e, &e->blk_ysplit, std::max(e->plan_x1.ysplit_halves, e->plan_x2.ysplit_halves)));
             DN_TRY(dev_alloc(e, &e->blk_partial, std::max(e->plan_x1.partial_floats, e->plan_x2.partial_floats)));
             DN_CUDA(cudaMemsetAsync(e->x1, 0, sizeof(__half) * e->plan_x1.x_halves, st));
@@ -908,7 +916,8 @@ int load_device(dnpeff_engine* e, int64_t n, int64_t m_full, int64_t k, const in
         trace.mark("extract, bucket, dense fill");
         if (dense) {
             dim3 sgrid((unsigned)e->plan_x1.m_tiles, (unsigned)(2 * e->plan_x2.m_tiles));
-            k_block_split<<<sgrid, 256, 0, st>>>(e->x1, e->x1_max, e->plan_x1.k_chunks, e->x2, e->x2_max, e->plan_x2.k_chunks);
+            k_block_split<<<sgrid, 256, 0, st>>>(e->x1, e->x1_max, e->x1_sum, e->plan_x1.k_chunks, e->x2, e->x2_max, e->x2_sum,
+                                                 e->plan_x2.k_chunks);
             DN_LAUNCH_CHECK();
             DN_COUNT_LAUNCH(1);
         }
@@ -1092,6 +1101,11 @@ int device_dot(dnpeff_engine* e, const float* a, const float* b, int64_t count, 
     return DNPEFF_OK;
 }
 
+// The stored entries behind x1 (`columns`: behind x2, whose rows are the popular columns).
+BlkValues popular_values(const dnpeff_engine* e, bool columns) {
+    return {nullptr, e->b_vals, e->b_col, e->a_rowptr, e->tail_off, e->n_tail_blocks + 1, columns};
+}
+
 // A*H^T: the popular columns through the tiled kernel (H tiles staged in shared
 // memory), then one launch per tail column block, each adding to AH, so that the
 // slice of H being gathered stays L2-resident.
@@ -1105,7 +1119,8 @@ int spmm_ah(dnpeff_engine* e, float* AH) {
     const int stride = e->n_tail_blocks + 1;
     if (e->x1) {
         // popular block on the tensor cores: AH = A_pop * H_pop (H's first n_hot rows)
-        DN_TRY(block_tc_launch(e->x1, e->x1_max, e->plan_x1, e->H, e->n, e->n_hot, ld, AH, e->blk_ysplit, e->y_max[0],
+        const BlkOperand x = {e->x1, e->x1_max, e->x1_sum, popular_values(e, false)};
+        DN_TRY(block_tc_launch(x, e->plan_x1, e->H, e->n, e->n_hot, ld, AH, e->W, e->blk_again, e->blk_ysplit, e->y_max[0],
                                e->y_max[1], e->blk_partial, e->d_err, e->st, e->opt_wait_limit));
         std::swap(e->y_max[0], e->y_max[1]);
         accumulate = 1;
@@ -1144,7 +1159,8 @@ int spmm_wa(dnpeff_engine* e) {
         return spmm_dispatch(csc_vals(e), csc_rows(e), e->c_colptr, e->ms, e->W, ld, e->WA, e->plan_csc, e->st);
     if (e->x2) {
         // popular columns on the tensor cores: WA[0, n_hot) = A_pop^T * W
-        DN_TRY(block_tc_launch(e->x2, e->x2_max, e->plan_x2, e->W, e->n_hot, e->n, ld, e->WA, e->blk_ysplit, e->y_max[0],
+        const BlkOperand x = {e->x2, e->x2_max, e->x2_sum, popular_values(e, true)};
+        DN_TRY(block_tc_launch(x, e->plan_x2, e->W, e->n_hot, e->n, ld, e->WA, e->H, e->blk_again, e->blk_ysplit, e->y_max[0],
                                e->y_max[1], e->blk_partial, e->d_err, e->st, e->opt_wait_limit));
         std::swap(e->y_max[0], e->y_max[1]);
     } else if (e->n_hot > 0) {
@@ -2232,16 +2248,22 @@ int dnpeff_op_block_product(const float* X, int64_t M, int64_t K, const float* Y
     DevBuf<float> partial;
     DevBuf<__half> xb, ysplit;
     DevBuf<uint32_t> maxima;  // of the rows of X, then of the columns of Y (two sets)
+    DevBuf<unsigned long long> sums;
+    DevBuf<unsigned char> again;
     DN_TRY(xb.alloc(p.x_halves));
     DN_TRY(ysplit.alloc(p.ysplit_halves));
     DN_TRY(partial.alloc(p.partial_floats));
     DN_TRY(maxima.alloc_zero(p.xmax_words + 2 * (size_t)r, st));
+    DN_TRY(sums.alloc(p.xmax_words));
+    DN_TRY(again.alloc_zero((size_t)M, st));
     int* err = nullptr;
     DN_TRY(op_err_word(&err));
     uint32_t* const ymax = maxima.p + p.xmax_words;
-    k_block_layout<<<(unsigned)(p.m_tiles * 16), 256, 0, st>>>(X, M, K, p.m_tiles, p.k_chunks, xb.p, maxima.p);
+    k_block_layout<<<(unsigned)(p.m_tiles * 16), 256, 0, st>>>(X, M, K, p.m_tiles, p.k_chunks, xb.p, maxima.p,
+                                                                   sums.p);
     DN_LAUNCH_CHECK();
-    DN_TRY(block_tc_launch(xb.p, maxima.p, p, Y, M, K, r, C, ysplit.p, ymax, ymax + r, partial.p, err, st));
+    const BlkOperand x = {xb.p, maxima.p, sums.p, {X, nullptr, nullptr, nullptr, nullptr, 0, false}};
+    DN_TRY(block_tc_launch(x, p, Y, M, K, r, C, nullptr, again.p, ysplit.p, ymax, ymax + r, partial.p, err, st));
     int s = op_check_err(err, st);
     DN_CUDA(cudaStreamSynchronize(st));  // the scratch buffers are released on return
     return s;

@@ -8,10 +8,15 @@
 //
 // Precision.  Every operand x, scaled by a power of two that brings the largest magnitude of its row of X
 // (its column of Y) into [2^14, 2^15), is split into hi = fp16(x) and lo = fp16((x - hi) * 2^11), both
-// rounded to nearest: within 2^-24 of x for what lies above 2^-29 of that largest value, and
-// within 2^-50 of it for what lies under.  hi*hi and hi*lo + lo*hi go to accumulators of their own, the
+// rounded to nearest: within 2^-24 of x while the scaled value is at least 2^-12 (a 2^-27th of the largest),
+// within 2^-36 (2^-51 of the largest) below.  hi*hi and hi*lo + lo*hi go to accumulators of their own, the
 // second counting 2^-11; lo*lo is left out.  Measured against float64, sums of 20000 terms: 1.1e-7 where a
 // quarter of X is stored (with tf32 halves, truncated, in one accumulator: 5.3e-7).
+// Values below 2^-12 ("faint") matter only where a sum consists of little else, and there they must not be
+// lost: a numerator that comes out zero would hold its factor entry at zero for good.  Rows of X and
+// columns of Y with faint values are marked, and where such a row or column meets a sum so small that the
+// representation could be off by 2^-23 of it, the row of C is computed again from the values themselves
+// (blk_faint, k_block_repair).
 //
 // Layouts.  X is split when the matrix is loaded (4 bytes per element, as fp32), in blocks of 128
 // rows x 64 K-values, block (tile, chunk) at (tile * k_chunks + chunk) * 32 KB: [hi | lo], each in the
@@ -92,17 +97,25 @@ __device__ __forceinline__ float blk_unscale(uint32_t max_bits) {
 }
 constexpr float kBlkLoScale = 2048.f;  // of the lo halves
 
-// v, a sum of products of scaled operands, with both scalings taken out, the smaller factor first: v is at
-// least about 1, so that neither step leaves the range of fp32 unless the result does.
-__device__ __forceinline__ float blk_unscaled(float v, uint32_t row_max, uint32_t col_max) {
-    const float a = blk_unscale(row_max), b = blk_unscale(col_max);
+// Marks in the sign bit of a maximum's word: the row (column) holds values other than zero that are below
+// kBlkFaint once they are scaled.
+constexpr uint32_t kBlkMark = 0x80000000u;
+constexpr float kBlkFaint = 1.f / 4096.f;
+
+// v, a product of scaled operands, with both scalings taken out: the smaller factor first, since v is at
+// least 1 or of no consequence (below) and neither step then leaves the range of fp32 unless the result does.
+__device__ __forceinline__ float blk_unscaled(float v, uint32_t row_word, uint32_t col_word) {
+    const float a = blk_unscale(row_word), b = blk_unscale(col_word);
     return v * fminf(a, b) * fmaxf(a, b);
 }
-__device__ __forceinline__ float4 blk_unscaled4(const float4& v, uint32_t row_max, const uint4& m) {
-    return make_float4(blk_unscaled(v.x, row_max, m.x), blk_unscaled(v.y, row_max, m.y), blk_unscaled(v.z, row_max, m.z),
-                       blk_unscaled(v.w, row_max, m.w));
+// Whether v, a scaled sum, may be off by more than 2^-23 of itself for what the halves do not hold.  A faint
+// value of Y is off by 2^-36 at most, one of X by 2^-35 (k_block_split) and meets 2^15 at most:
+// 2^-36 * sum |x| + 2^-35 * 2^15 * (faint values of the row) in all, that is 2^-36 times `row_sum`, which
+// k_block_split and k_block_layout add up as sum |x| + 2^16 * (faint values).
+constexpr unsigned long long kBlkFaintWeight = 65536;
+__device__ __forceinline__ bool blk_faint(float v, uint32_t row_word, uint32_t col_word, float row_sum) {
+    return ((row_word | col_word) & kBlkMark) && fabsf(v) < row_sum * (1.f / 8192.f);
 }
-
 // Two values times s as fp16 pairs: hi, and lo (s2 = s * 2^11).
 __device__ __forceinline__ void blk_split2(float x, float y, float s, float s2, uint32_t& hi, uint32_t& lo) {
     const __half2 h = __floats2half2_rn(x * s, y * s);
@@ -117,6 +130,20 @@ __device__ __forceinline__ void blk_split8(const float (&v)[8], uint32_t max_bit
     blk_split2(v[2], v[3], s, s2, hi.y, lo.y);
     blk_split2(v[4], v[5], s, s2, hi.z, lo.z);
     blk_split2(v[6], v[7], s, s2, hi.w, lo.w);
+}
+
+// How many of eight values are faint under the scale s.
+__device__ __forceinline__ uint32_t blk_count_faint(const float (&v)[8], float s) {
+    uint32_t n = 0;
+#pragma unroll
+    for (int t = 0; t < 8; t++) n += v[t] != 0.f && fabsf(v[t] * s) < kBlkFaint ? 1u : 0u;
+    return n;
+}
+
+// The smallest lo half for values other than zero that both halves would lose.
+__device__ __forceinline__ uint32_t blk_lost2(float x, float y, uint32_t hi, uint32_t lo) {
+    const uint32_t some = hi | lo;
+    return (x != 0.f && !(some & 0x7fffu) ? 1u : 0u) | (y != 0.f && !(some & 0x7fff0000u) ? 0x10000u : 0u);
 }
 
 // ymax[c] = bits of the largest magnitude in column c of Y (K rows, r columns); zero before.
@@ -155,9 +182,9 @@ k_col_max(const float* __restrict__ Y, int64_t K, int r, uint32_t* __restrict__ 
 
 // Y (K rows, r columns) in panels of pn columns -> per panel and chunk of 64 K-values
 // [hi pn*64 | lo pn*64] fp16 in core matrices of 8 columns x 8 K-values; rows K..64*k_chunks are zero.
-// One thread per (panel, K octet, column).  Clears `clear` (r words) for the next product.
-__global__ void k_split_y(const float* __restrict__ Y, int64_t K, int r, int pn, int64_t k_chunks,
-                          const uint32_t* __restrict__ ymax, uint32_t* __restrict__ clear, __half* __restrict__ Ysplit) {
+// One thread per (panel, K octet, column).  Marks columns with faint values.  Clears `clear` (r words) for the next product.
+__global__ void k_split_y(const float* __restrict__ Y, int64_t K, int r, int pn, int64_t k_chunks, uint32_t* ymax,
+                          uint32_t* __restrict__ clear, __half* __restrict__ Ysplit) {
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     grid_wait();
     if (idx < r) clear[idx] = 0u;
@@ -168,19 +195,46 @@ __global__ void k_split_y(const float* __restrict__ Y, int64_t K, int r, int pn,
 #pragma unroll
     for (int j = 0; j < 8; j++) v[j] = ko * 8 + j < K ? Y[(ko * 8 + j) * r + col] : 0.f;
     uint4 hi, lo;
-    blk_split8(v, ymax[col], hi, lo);
+    const uint32_t most = ymax[col];
+    blk_split8(v, most, hi, lo);
+    if (blk_count_faint(v, blk_scale(most)) && !(__ldcg(ymax + col) & kBlkMark)) atomicOr(ymax + col, kBlkMark);
     const int64_t c = ko / 8;
     __half* base = Ysplit + (panel * k_chunks + c) * (2 * 64) * pn + blk_canon(n, (int)(ko % 8) * 8);
     *(uint4*)base = hi;
     *(uint4*)(base + 64 * pn) = lo;
 }
 
-// r: columns of a panel.  direct: C, with row stride ldc and its scaling (row_max, col_max) -- or null.
+__device__ __forceinline__ float4 blk_unscaled4(const float4& v, uint32_t row_word, const uint4& m) {
+    return make_float4(blk_unscaled(v.x, row_word, m.x), blk_unscaled(v.y, row_word, m.y), blk_unscaled(v.z, row_word, m.z),
+                       blk_unscaled(v.w, row_word, m.w));
+}
+// Whether one of four sums at `at` wants computing again.
+__device__ __forceinline__ bool blk_again(const float4& v, uint32_t row_word, const uint4& m, float row_sum,
+                                          const float* __restrict__ keep, int64_t at) {
+    const bool a = blk_faint(v.x, row_word, m.x, row_sum), b = blk_faint(v.y, row_word, m.y, row_sum),
+               c = blk_faint(v.z, row_word, m.z, row_sum), d = blk_faint(v.w, row_word, m.w, row_sum);
+    if (!(a || b || c || d)) return false;
+    if (!keep) return true;
+    const float4 k = *(const float4*)(keep + at);
+    return (a && k.x != 0.f) || (b && k.y != 0.f) || (c && k.z != 0.f) || (d && k.w != 0.f);
+}
+
+// What the last step of a product needs beside its sums: the operands' scaling, and where rows that want
+// computing again are noted.  keep (or null): the factor whose numerators C holds, of C's shape; where it is
+// zero, so is its update whatever the numerator.
+struct BlkFinish {
+    const uint32_t* row_max;
+    const uint32_t* col_max;
+    const unsigned long long* row_sum;
+    const float* keep;
+    unsigned char* again;  // one byte per row of C
+};
+
+// r: columns of a panel.  direct: C, with row stride ldc -- or null, and `fin` is not used.
 __global__ void __launch_bounds__(kBlkThreads, 1)
 k_block_tc(const __half* __restrict__ X, int64_t m_tiles, int64_t k_chunks, const __half* __restrict__ Ysplit, int r,
            int panels, int n_split, int64_t chunks_per_split, int stages, float* __restrict__ partial, uint32_t buf_cols,
-           float* __restrict__ direct, int64_t rows, int ldc, const uint32_t* __restrict__ row_max,
-           const uint32_t* __restrict__ col_max, uint32_t wait_limit, int* __restrict__ err) {
+           float* __restrict__ direct, int64_t rows, int ldc, const BlkFinish fin, uint32_t wait_limit, int* __restrict__ err) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t full[kBlkStages], free_[kBlkStages];
     __shared__ __align__(8) uint64_t acc_done[2], acc_free[2];
@@ -259,7 +313,12 @@ k_block_tc(const __half* __restrict__ X, int64_t m_tiles, int64_t k_chunks, cons
                 const int col0 = cur.panel * r + ch * 64;
                 const bool store = !direct || row < rows;
                 uint32_t row_word = 0u;
-                if (direct && store) row_word = __ldg(row_max + row);
+                float row_sum = 0.f;
+                bool again = false;
+                if (direct && store) {
+                    row_word = __ldg(fin.row_max + row);
+                    row_sum = (float)__ldg(fin.row_sum + row);
+                }
                 float* dst = direct ? direct + row * ldc + col0
                                     : partial + (((cur.split * panels + cur.panel) * m_tiles + cur.tile) * 128 + xrow) * (int64_t)r + ch * 64;
 #pragma unroll
@@ -274,13 +333,16 @@ k_block_tc(const __half* __restrict__ X, int64_t m_tiles, int64_t k_chunks, cons
                         for (int j = 0; j < 16; j += 4) {
                             float4 x = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
                             if (direct) {
-                                const uint4 m = __ldg((const uint4*)(col_max + col0 + g * 16 + j));
+                                const int col = col0 + g * 16 + j;
+                                const uint4 m = __ldg((const uint4*)(fin.col_max + col));
+                                again = again || blk_again(x, row_word, m, row_sum, fin.keep, row * ldc + col);
                                 x = blk_unscaled4(x, row_word, m);
                             }
                             if (store) *(float4*)(dst + g * 16 + j) = x;
                         }
                     }
                 }
+                if (again) fin.again[row] = 1;
                 tc_fence_before();
                 if (lane == 0) mbar_arrive(&cross_free);
 #pragma unroll
@@ -398,13 +460,19 @@ __global__ void k_fill_blocks(const float* __restrict__ vals, const int32_t* __r
 
 // A block of X1 from fp32 into its halves, in place, and its transpose into X2.  Block (it, c1) of the
 // grid takes rows 128 it.. and columns 64 c1.. through shared memory; blocks past the last chunk of X1 write
-// the zeros that pad X2's last tile (X2 needs no clearing).  xmax1, xmax2: largest magnitudes of the rows of
-// either.  Reads 4 bytes and writes 8 per element.  256 threads; 8 consecutive ones write a core matrix.
+// the zeros that pad X2's last tile (X2 needs no clearing).  max1, max2: largest magnitudes of the rows of
+// either, marked here; sum1, sum2 (zero before): their row_sum (blk_faint), in whole numbers, so that the
+// order of the additions does not matter.  Reads 4 bytes and writes 8 per element.  256 threads; 8
+// consecutive ones write a core matrix.
+// A value that both halves in X2 would lose is left there as their smallest, 2^-35: k_block_repair
+// has to see that there is one, and looks it up.
 __global__ void __launch_bounds__(256)
-k_block_split(__half* __restrict__ X1, const uint32_t* __restrict__ xmax1, int64_t chunks1, __half* __restrict__ X2,
-              const uint32_t* __restrict__ xmax2, int64_t chunks2) {
+k_block_split(__half* __restrict__ X1, uint32_t* max1, unsigned long long* sum1, int64_t chunks1, __half* __restrict__ X2,
+              uint32_t* max2, unsigned long long* sum2, int64_t chunks2) {
     __shared__ float sq[128][kBlkKC + 1];
+    __shared__ uint32_t part1[2][128], part2[4][kBlkKC];  // of the sums, by octets that one warp holds
     const int64_t it = blockIdx.x, c1 = blockIdx.y;
+    const int lane = threadIdx.x & 31;
     __half* const x1 = X1 + (it * chunks1 + c1) * kBlkHalves;
     const bool stored = c1 < chunks1;
 #pragma unroll
@@ -415,6 +483,17 @@ k_block_split(__half* __restrict__ X1, const uint32_t* __restrict__ xmax1, int64
         d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
     }
     __syncthreads();
+    // of the eight values of a lane and of the lanes 8, 16 and 24 further on
+    auto sum_of_octets = [&](const float (&v)[8], uint32_t word) {
+        const float s = blk_scale(word);
+        float sum = 0.f;
+#pragma unroll
+        for (int t = 0; t < 8; t++) sum += fabsf(v[t] * s);
+        // 24 bits of sum (32 values below 2^15, rounded up by octets), then the faint ones
+        uint32_t q = min(__float2uint_ru(sum), 8u << 15) + (blk_count_faint(v, s) << 24);
+        q += __shfl_xor_sync(0xffffffffu, q, 8);
+        return q + __shfl_xor_sync(0xffffffffu, q, 16);
+    };
     if (stored) {
 #pragma unroll
         for (int e = threadIdx.x; e < 128 * 8; e += 256) {  // (row, octet of columns)
@@ -423,57 +502,246 @@ k_block_split(__half* __restrict__ X1, const uint32_t* __restrict__ xmax1, int64
 #pragma unroll
             for (int t = 0; t < 8; t++) v[t] = sq[row][8 * ko + t];
             uint4 hi, lo;
-            blk_split8(v, __ldg(xmax1 + it * 128 + row), hi, lo);
+            const uint32_t word = __ldcg(max1 + it * 128 + row);
+            blk_split8(v, word, hi, lo);
             *(uint4*)(x1 + blk_canon(row, 8 * ko)) = hi;
             *(uint4*)(x1 + kBlkHalf + blk_canon(row, 8 * ko)) = lo;
+            const uint32_t q = sum_of_octets(v, word);
+            if (lane < 8) part1[ko >> 2][row] = q;
         }
     }
 #pragma unroll
     for (int e = threadIdx.x; e < 64 * 16; e += 256) {  // (column, octet of rows)
         const int ko = (e >> 3) & 7, io = ko + 8 * (e >> 9), j = ((e >> 6) & 7) * 8 + (e & 7);
         const int64_t c2 = 2 * it + (io >> 3);
-        if (c2 >= chunks2) continue;
         float v[8];
 #pragma unroll
         for (int t = 0; t < 8; t++) v[t] = sq[8 * io + t][j];
         const int row2 = (int)(c1 & 1) * 64 + j;
+        const uint32_t word = __ldcg(max2 + (c1 >> 1) * 128 + row2);
+        const uint32_t q = sum_of_octets(v, word);
+        if (lane < 8) part2[io >> 2][j] = q;
+        if (c2 >= chunks2) continue;
         uint4 hi, lo;
-        blk_split8(v, __ldg(xmax2 + (c1 >> 1) * 128 + row2), hi, lo);
+        blk_split8(v, word, hi, lo);
+        lo.x |= blk_lost2(v[0], v[1], hi.x, lo.x);
+        lo.y |= blk_lost2(v[2], v[3], hi.y, lo.y);
+        lo.z |= blk_lost2(v[4], v[5], hi.z, lo.z);
+        lo.w |= blk_lost2(v[6], v[7], hi.w, lo.w);
         __half* const x2 = X2 + ((c1 >> 1) * chunks2 + c2) * kBlkHalves + blk_canon(row2, 8 * ko);
         *(uint4*)x2 = hi;
         *(uint4*)(x2 + kBlkHalf) = lo;
     }
+    __syncthreads();
+    if (!stored) return;
+    const int t = threadIdx.x;
+    if (t < 128 + kBlkKC) {
+        const bool row = t < 128;
+        const int j = t - 128;
+        const int64_t at = row ? it * 128 + t : c1 * kBlkKC + j;
+        const uint32_t parts[4] = {row ? part1[0][t] : part2[0][j], row ? part1[1][t] : part2[1][j], row ? 0u : part2[2][j],
+                                   row ? 0u : part2[3][j]};
+        unsigned long long q = 0;
+        bool faint = false;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            q += (parts[k] & 0xffffffu) + (parts[k] >> 24) * kBlkFaintWeight;
+            faint = faint || (parts[k] >> 24);
+        }
+        if (q) atomicAdd((row ? sum1 : sum2) + at, q);
+        if (faint && !(__ldcg((row ? max1 : max2) + at) & kBlkMark)) atomicOr((row ? max1 : max2) + at, kBlkMark);
+    }
 }
 
 // A row-major dense X (M x K) split into the blocked layout of k_block_tc (zero
-// padding included): one warp per row of the blocked matrix.  xmax[row] as in k_fill_blocks.
-__global__ void k_block_layout(const float* __restrict__ X, int64_t M, int64_t K, int64_t m_tiles,
-                               int64_t k_chunks, __half* __restrict__ Xb, uint32_t* __restrict__ xmax) {
+// padding included): one warp per row of the blocked matrix.  xmax, xsum: as k_block_split leaves them.
+__global__ void k_block_layout(const float* __restrict__ X, int64_t M, int64_t K, int64_t m_tiles, int64_t k_chunks,
+                               __half* __restrict__ Xb, uint32_t* __restrict__ xmax, unsigned long long* __restrict__ xsum) {
     const int lane = threadIdx.x & 31;
     const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (i >= m_tiles * 128) return;
     uint32_t most = 0u;
     for (int64_t k = lane; i < M && k < K; k += 32) most = max(most, __float_as_uint(X[i * K + k]) & 0x7fffffffu);
     most = __reduce_max_sync(0xffffffffu, most);
-    if (lane == 0) xmax[i] = most;
     __half* const x = Xb + (i >> 7) * k_chunks * kBlkHalves;
+    const float s = blk_scale(most);
+    unsigned long long sum = 0, faint = 0;
     for (int64_t ko = lane; ko < k_chunks * 8; ko += 32) {
-        float v[8];
+        float v[8], octet = 0.f;
 #pragma unroll
-        for (int t = 0; t < 8; t++) v[t] = i < M && ko * 8 + t < K ? X[i * K + ko * 8 + t] : 0.f;
+        for (int t = 0; t < 8; t++) {
+            v[t] = i < M && ko * 8 + t < K ? X[i * K + ko * 8 + t] : 0.f;
+            octet += fabsf(v[t] * s);
+        }
+        sum += __float2uint_ru(octet);
+        faint += blk_count_faint(v, s);
         uint4 hi, lo;
         blk_split8(v, most, hi, lo);
         __half* const d = x + (ko >> 3) * kBlkHalves + blk_canon((int)(i & 127), (int)(ko & 7) * 8);
         *(uint4*)d = hi;
         *(uint4*)(d + kBlkHalf) = lo;
     }
+    sum += faint * kBlkFaintWeight;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        faint += __shfl_xor_sync(0xffffffffu, faint, o);
+    }
+    if (lane == 0) {
+        xmax[i] = most | (faint ? kBlkMark : 0u);
+        xsum[i] = sum;
+    }
+}
+
+// Where the values of X are kept as they are: as a row-major matrix, or as the stored entries of the
+// popular columns in the rows of A, that is the rows of X or (`columns`) its columns.
+struct BlkValues {
+    const float* dense;        // K values per row of X, or null:
+    const float* vals;
+    const int32_t* col;        // internal column ids
+    const int64_t* rowptr;
+    const uint32_t* hot_len;   // entries of a row of A in popular columns (they come first), every `stride` words
+    int stride;
+    bool columns;
+};
+
+// The rows of C = X * Y whose byte in `again` is set (it is cleared), from the values of X as they are,
+// products and sums in double: what the halves lose of faint values is in these rows
+// too much (blk_faint).  Almost always there are none, and the launch costs a product 3.5 us (3001 x 100003,
+// rank 50).  Where it has to work it is bound by latency: every popular column of 20000 x 4194304 at rank 128 computed
+// again takes 75 ms, the sparse product of the same entries 12.  It stays that way since entries that are
+// this small only last a few updates.  With `columns` the stored entries of a row of X are found
+// through its halves, and the faint ones among them in the row of A.
+constexpr int kRepairThreads = 256, kRepairBatch = 8;
+__global__ void __launch_bounds__(kRepairThreads, 2)
+k_block_repair(const __half* __restrict__ X, const uint32_t* __restrict__ xmax, int64_t k_chunks, const BlkValues ex,
+               const float* __restrict__ Y, int64_t M, int64_t K, int r, float* __restrict__ C, unsigned char* __restrict__ again) {
+    constexpr int kWarps = kRepairThreads / 32;
+    __shared__ int64_t list[kRepairThreads];
+    __shared__ int listed;
+    __shared__ double sums[kWarps][512];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    grid_wait();
+    const int quads = r >> 2;
+    // 32 consecutive rows per warp and round
+    for (int64_t g0 = (int64_t)blockIdx.x * kWarps; g0 * 32 < M; g0 += (int64_t)gridDim.x * kWarps) {
+        if (tid == 0) listed = 0;
+        __syncthreads();
+        const int64_t mine = (g0 + w) * 32 + lane;
+        if (mine < M && again[mine]) {
+            again[mine] = 0;
+            list[atomicAdd(&listed, 1)] = mine;  // (in any order: the rows do not depend on one another)
+        }
+        __syncthreads();
+        const int n = listed;
+        for (int l = 0; l < n; l++) {
+            const int64_t i = list[l];
+            double acc[4][4];
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+#pragma unroll
+                for (int t = 0; t < 4; t++) acc[q][t] = 0.0;
+            int64_t beg = 0, end = K;
+            if (!ex.dense && !ex.columns) {
+                beg = ex.rowptr[i];
+                end = beg + ex.hot_len[i * ex.stride];
+            }
+            const float back = blk_unscale(xmax[i]);
+            for (int64_t p0 = beg + w * 32; p0 < end; p0 += kRepairThreads) {
+                const int64_t p = p0 + lane;
+                int64_t k = p;
+                float v = 0.f;
+                if (p < end) {
+                    if (ex.dense) {
+                        v = ex.dense[i * K + p];
+                    } else if (!ex.columns) {
+                        k = ex.col[p];
+                        v = ex.vals[p];
+                    } else {
+                        const __half* x = X + ((i >> 7) * k_chunks + (p >> 6)) * kBlkHalves + blk_canon((int)(i & 127), (int)(p & 63));
+                        v = fmaf(__half2float(x[kBlkHalf]), 1.f / kBlkLoScale, __half2float(x[0]));
+                    }
+                }
+                if (!ex.dense && ex.columns) {
+                    uint32_t ask = __ballot_sync(0xffffffffu, v != 0.f && fabsf(v) < kBlkFaint);
+                    v *= back;
+                    while (ask) {
+                        const int src = __ffs(ask) - 1;
+                        ask &= ask - 1;
+                        const int64_t row = __shfl_sync(0xffffffffu, k, src), first = ex.rowptr[row];
+                        const int64_t last = first + ex.hot_len[row * ex.stride];
+                        for (int64_t q = first; q < last; q += 32 * kRepairBatch) {
+                            int found = -1;
+#pragma unroll
+                            for (int b = 0; b < kRepairBatch; b++) {
+                                const int64_t at = q + 32 * b + lane;
+                                if (at < last && ex.col[at] == i) found = b;
+                            }
+                            const uint32_t hit = __ballot_sync(0xffffffffu, found >= 0);
+                            if (!hit) continue;
+                            const int by = __ffs(hit) - 1;
+                            const int b = __shfl_sync(0xffffffffu, found, by);
+                            if (lane == src) v = ex.vals[q + 32 * b + by];
+                            break;
+                        }
+                    }
+                }
+                uint32_t live = __ballot_sync(0xffffffffu, v != 0.f);
+                while (live) {
+                    double x[kRepairBatch];  // that many entries at a time, so that their rows of Y are on the way together
+                    int64_t at[kRepairBatch];
+                    int m = 0;
+#pragma unroll
+                    for (int b = 0; b < kRepairBatch; b++) {
+                        const int src = live ? __ffs(live) - 1 : 0;
+                        x[b] = (double)__shfl_sync(0xffffffffu, v, src);
+                        at[b] = __shfl_sync(0xffffffffu, k, src) * quads;
+                        m += live ? 1 : 0;
+                        live &= live - 1;
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        if (32 * q >= quads) continue;
+                        const int c = lane + 32 * q;
+                        float4 f[kRepairBatch];
+#pragma unroll
+                        for (int b = 0; b < kRepairBatch; b++) {
+                            f[b] = make_float4(0.f, 0.f, 0.f, 0.f);
+                            if (b < m && c < quads) f[b] = __ldg((const float4*)Y + at[b] + c);
+                        }
+#pragma unroll
+                        for (int b = 0; b < kRepairBatch; b++) {
+                            if (b >= m) continue;
+                            acc[q][0] = fma(x[b], (double)f[b].x, acc[q][0]);
+                            acc[q][1] = fma(x[b], (double)f[b].y, acc[q][1]);
+                            acc[q][2] = fma(x[b], (double)f[b].z, acc[q][2]);
+                            acc[q][3] = fma(x[b], (double)f[b].w, acc[q][3]);
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (lane + 32 * q < quads)
+#pragma unroll
+                    for (int t = 0; t < 4; t++) sums[w][4 * (lane + 32 * q) + t] = acc[q][t];
+            __syncthreads();
+            for (int c = tid; c < r; c += kRepairThreads) {
+                double t = sums[0][c];
+#pragma unroll
+                for (int k = 1; k < kWarps; k++) t += sums[k][c];
+                C[i * r + c] = (float)t;
+            }
+            __syncthreads();
+        }
+        __syncthreads();  // (the list is read before it is started anew)
+    }
 }
 
 // out[i][:] (rows i < rows, r4 float4 each) = sum over splits s (in index order) of partial[s][panel][i][:],
 // with the operands' scaling taken out.
 __global__ void k_block_reduce(const float* __restrict__ partial, int n_split, int64_t rows_pad, int64_t rows,
-                               int r4, int pn4, const uint32_t* __restrict__ row_max, const uint32_t* __restrict__ col_max,
-                               float4* __restrict__ out) {
+                               int r4, int pn4, const BlkFinish fin, float4* __restrict__ out) {
     int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     grid_wait();
     if (idx >= rows * r4) return;
@@ -485,7 +753,10 @@ __global__ void k_block_reduce(const float* __restrict__ partial, int n_split, i
         float4 b = p[(int64_t)s * rows_pad * r4];
         a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
     }
-    out[idx] = blk_unscaled4(a, __ldg(row_max + i), __ldg((const uint4*)col_max + c));
+    const uint32_t row_word = __ldg(fin.row_max + i);
+    const uint4 m = __ldg((const uint4*)fin.col_max + c);
+    if (blk_again(a, row_word, m, (float)__ldg(fin.row_sum + i), fin.keep, 4 * idx)) fin.again[i] = 1;
+    out[idx] = blk_unscaled4(a, row_word, m);
 }
 
 // Ranks up to 128 in one panel; 256, 384 and 512 as panels of 128 columns of Y and C.
@@ -523,11 +794,19 @@ inline BlockTcPlan block_tc_plan(int64_t M, int64_t K, int r) {
     return p;
 }
 
-// C (M x r, overwritten) = X * Y.  X in the blocked layout above with its xmax, Y row-major K x r.
+// X of a product: its blocks, the words and sums of its rows (BlkFinish), and its values.
+struct BlkOperand {
+    const __half* blocks;
+    const uint32_t* max;
+    const unsigned long long* sum;
+    BlkValues values;
+};
+
+// C (M x r, overwritten) = X * Y.  Y row-major K x r.  keep: as in BlkFinish.  again: M bytes, zero before and after.
 // ymax: r words, zero before the call; ymax_next: r words that are zero after it, for the next one.
-inline int block_tc_launch(const __half* X, const uint32_t* xmax, const BlockTcPlan& p, const float* Y, int64_t M,
-                           int64_t K, int r, float* C, __half* ysplit, uint32_t* ymax, uint32_t* ymax_next, float* partial,
-                           int* err, cudaStream_t st, uint32_t wait_limit = kTiledSpinLimit) {
+inline int block_tc_launch(const BlkOperand& X, const BlockTcPlan& p, const float* Y, int64_t M, int64_t K, int r, float* C,
+                           const float* keep, unsigned char* again, __half* ysplit, uint32_t* ymax, uint32_t* ymax_next,
+                           float* partial, int* err, cudaStream_t st, uint32_t wait_limit = kTiledSpinLimit) {
     if (M <= 0) return DNPEFF_OK;
     const int pn = block_tc_panel(r);
     const size_t stage = (size_t)kBlkHalves * 2 + (size_t)pn * kBlkKC * 4;
@@ -540,14 +819,16 @@ inline int block_tc_launch(const __half* X, const uint32_t* xmax, const BlockTcP
                              256, 0, st, Y, K, r, ymax));
     DN_TRY(launch_overlapped(k_split_y, dim3((unsigned)ceil_div(p.k_chunks * 8 * r, 256)), 256, 0, st, Y, K, r, pn, p.k_chunks,
                              ymax, ymax_next, ysplit));
+    const BlkFinish fin = {X.max, ymax, X.sum, keep, again};
     const int64_t items = p.m_tiles * p.n_split * p.panels;
-    DN_TRY(launch_overlapped(k_block_tc, dim3((unsigned)std::min<int64_t>(items, (int64_t)kNumSMs)), kBlkThreads, smem, st, X,
+    DN_TRY(launch_overlapped(k_block_tc, dim3((unsigned)std::min<int64_t>(items, (int64_t)kNumSMs)), kBlkThreads, smem, st, X.blocks,
                              p.m_tiles, p.k_chunks, ysplit, pn, p.panels, p.n_split, p.chunks_per_split, stages, partial,
-                             tc_tmem_cols(pn), p.n_split > 1 ? (float*)nullptr : C, M, r, xmax, ymax, wait_limit, err));
+                             tc_tmem_cols(pn), p.n_split > 1 ? (float*)nullptr : C, M, r, fin, wait_limit, err));
     if (p.n_split > 1)
         DN_TRY(launch_overlapped(k_block_reduce, dim3((unsigned)ceil_div(M * (r / 4), 256)), 256, 0, st, partial, p.n_split,
-                                 p.m_tiles * 128, M, r / 4, pn / 4, xmax, ymax, (float4*)C));
-    return DNPEFF_OK;
+                                 p.m_tiles * 128, M, r / 4, pn / 4, fin, (float4*)C));
+    return launch_overlapped(k_block_repair, dim3((unsigned)std::min<int64_t>(ceil_div(M, kRepairThreads), 2 * kNumSMs)), kRepairThreads, 0,
+                             st, X.blocks, X.max, p.k_chunks, X.values, Y, M, K, r, C, again);
 }
 
 }  // namespace dnpeff

@@ -355,6 +355,77 @@ def test_op_block_product_opposite_scales(torch_cuda, M, K, r, x_size, y_size):
     assert np.all(np.abs(C_.cpu().numpy() - want) <= 2e-6 * want)
 
 
+@pytest.mark.parametrize("M,K,r", [(1, 64, 32), (127, 640, 128), (300, 2000, 96), (300, 2000, 512), (1000, 70, 256)])
+def test_op_block_product_faint_values(torch_cuda, M, K, r):
+    """Values far below the largest of their row of X or column of Y (down to 1e-20 of it), in sums that
+    consist of nothing else: the tolerance is relative to every single sum, as for ordinary values.  A
+    third of the rows of X is stored only where half of the columns of Y are faint; one value in ten of X is
+    faint; columns of Y that are faint, or zero, all over."""
+    from npeff_ref_b200._lib import lib, check
+    torch = torch_cuda
+    rng = np.random.default_rng(7 * M + K + r)
+    half = K // 2
+    X = rng.uniform(0.1, 1.0, (M, K)) * (rng.random((M, K)) < 0.3)
+    X *= np.where(rng.random((M, K)) < 0.1, 10.0 ** rng.uniform(-15, -8, (M, K)), 1.0)
+    X[0::3, half:] = 0.0
+    X[1::3, 0] = 1e-13    # the only partner of column 3 below in these rows
+    Y = rng.uniform(0.1, 1.0, (K, r))
+    Y[:half, 0::2] *= 10.0 ** rng.uniform(-20, -6, (half, len(range(0, r, 2))))
+    Y[:, 4] *= 1e-20
+    Y[:, 5] = 0.0
+    Y[1:half, 3] = 0.0
+    Y[half:, 3] = 0.0
+    X, Y = X.astype(np.float32), Y.astype(np.float32)
+    want = X.astype(np.float64) @ Y.astype(np.float64)
+    dX, dY = _dev(torch, X), _dev(torch, Y)
+    C_ = torch.full((M, r), float("nan"), device="cuda")
+    for _ in range(2):
+        check(lib().dnpeff_op_block_product(dX.data_ptr(), M, K, dY.data_ptr(), r, C_.data_ptr(),
+                                            torch.cuda.current_stream().cuda_stream))
+        torch.cuda.synchronize()
+        got = C_.cpu().numpy()
+        assert np.all(np.abs(got - want) <= 2e-6 * want)
+
+
+@pytest.mark.parametrize("n,m,r", [(300, 500, 32), (300, 3000, 100), (1500, 400, 256)])
+def test_faint_factor_entries_keep_their_numerators(torch_cuda, n, m, r):
+    """Two groups of examples and columns that share no entry, with the odd components 1e-16 of their
+    largest in the second: every entry of both products that such a component gets there is a sum of
+    faint values.  One update of W and of H, each entry relative to itself (a numerator that came out zero
+    would end the entry for good), where all columns are popular and some entries of A are faint too."""
+    from npeff_ref_b200 import MuNmfParams
+    rng = np.random.default_rng(n + m + r)
+    A = rng.uniform(0.1, 1.0, (n, m)) * (rng.random((n, m)) < 0.3)
+    A *= np.where(rng.random((n, m)) < 0.05, 10.0 ** rng.uniform(-15, -9, (n, m)), 1.0)
+    A[:n // 2, m // 2:] = 0.0
+    A[n // 2:, :m // 2] = 0.0
+    A = A.astype(np.float32)
+    rowptr = np.zeros(n + 1, dtype=np.int64)
+    rowptr[1:] = np.cumsum((A != 0).sum(1))
+    colind = np.nonzero(A)[1].astype(np.int32)
+    vals = A[A != 0]
+    W0, H0 = rng.uniform(0.1, 1.0, (n, r)), rng.uniform(0.1, 1.0, (r, m))
+    W0[n // 2:, 1::2] *= 1e-16
+    H0[1::2, m // 2:] *= 1e-16
+    W0, H0 = W0.astype(np.float32), H0.astype(np.float32)
+    v, c, rp, n2o = O.prune_columns(vals, colind, rowptr, m, 1)
+    assert len(n2o) == m
+    eps = 1e-12
+    with _engine(MuNmfParams(rank=r, eps=eps)) as eng:
+        eng.set_csr(n, m, vals, colind, rowptr, 0, None, 1)
+        assert eng.layout()[0] == m        # every column is popular: the dense block is all there is
+        eng.init_factors(W0, H0)
+        eng.step_w()
+        W1 = eng.load_w_to_host()
+        eng.init_factors(W0, H0)
+        eng.step_h()
+        H1 = eng.load_h_to_host()
+    Wo, Ho = O.step_w(v, c, rp, m, W0, H0, eps), O.step_h(v, c, rp, m, W0, H0, eps)
+    assert Wo[n // 2:, 1::2].min() > 0 and Ho[1::2, m // 2:].min() > 0
+    assert np.all(np.abs(W1 - Wo) <= 1e-5 * Wo)
+    assert np.all(np.abs(H1 - Ho) <= 1e-5 * Ho)
+
+
 # ---------------------------------------------------------------------------
 CASES = [
     # n, m, k, r, iters, eps
