@@ -100,6 +100,10 @@ int dnpeff_destroy(dnpeff_engine* eng);
  *                       between the blocks of the small-problem kernel,
  *                       gives up (default 2^24); the kernel then leaves cleanly and the
  *                       next call that reads the engine's status returns DNPEFF_ERR_CUDA
+ *   "refuse_cooperative" 1: the launch of the small-problem kernel, whose blocks must all
+ *                       be on the GPU together, is treated as refused, as the runtime
+ *                       does where the process may use only some of the SMs (test hook);
+ *                       the kernels for larger problems then make the iterations
  * Unknown names fail with DNPEFF_ERR_INVALID. */
 int dnpeff_set_option(dnpeff_engine* eng, const char* name, int64_t value);
 

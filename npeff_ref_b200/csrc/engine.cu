@@ -159,6 +159,7 @@ struct dnpeff_engine {
     int opt_popular_divisor = 0;
     uint32_t opt_wait_limit = kTiledSpinLimit;
     bool opt_keep_csr = false;
+    bool opt_refuse_cooperative = false;
 };
 
 namespace {
@@ -1254,7 +1255,8 @@ bool small_problem(const dnpeff_engine* e) {
     return small_pays(e->nnz, e->n + e->ms, (e->p.rank + 3) / 4, e->ld);
 }
 
-int run_small(dnpeff_engine* e, int iters) {
+// *made: iterations that were made; fewer than asked for where the launch was refused.
+int run_small(dnpeff_engine* e, int iters, int* made) {
     ArenaScope arena_scope(&e->arena);
     const int ld = e->ld;
     DN_TRY(build_csc(e, true));
@@ -1284,9 +1286,11 @@ int run_small(dnpeff_engine* e, int iters) {
     a.barrier = e->small_barrier;
     a.wait_limit = e->opt_wait_limit;
     a.err = e->d_err;
-    for (int done = 0; done < iters; done += kSmallIters) {
-        a.iters = std::min(kSmallIters, iters - done);
-        DN_TRY(small_launch(a, ld, e->st));
+    for (*made = 0; *made < iters; *made += a.iters) {
+        a.iters = std::min(kSmallIters, iters - *made);
+        bool launched = false;
+        DN_TRY(small_launch(a, ld, e->st, e->opt_refuse_cooperative, &launched));
+        if (!launched) break;
     }
     return DNPEFF_OK;
 }
@@ -1530,6 +1534,8 @@ int dnpeff_set_option(dnpeff_engine* e, const char* name, int64_t value) {
         e->opt_popular_divisor = (int)value;
     } else if (!strcmp(name, "keep_canonical_csr")) {
         e->opt_keep_csr = value != 0;
+    } else if (!strcmp(name, "refuse_cooperative")) {
+        e->opt_refuse_cooperative = value != 0;
     } else if (!strcmp(name, "wait_limit")) {
         e->opt_wait_limit = value == 0 || value > kTiledSpinLimit ? kTiledSpinLimit : (uint32_t)value;
     } else {
@@ -2058,18 +2064,22 @@ int dnpeff_run_steps(dnpeff_engine* e, int32_t first_step, int32_t iters, int32_
         return fail(DNPEFF_ERR_INVALID, "sharded engine without a communicator: call dnpeff_comm_init");
     if (first_step < 0) return fail(DNPEFF_ERR_INVALID, "negative first step");
     auto t0 = std::chrono::high_resolution_clock::now();
-    const bool small = small_problem(e) && iters > 1;
+    bool small = small_problem(e) && iters > 1;
     for (int step = first_step; step < first_step + iters; step++) {
+        int made = 0;
         if (small) {
             // as far as the next log line
             int stretch = first_step + iters - step;
             if (log_every > 0) stretch = std::min(stretch, log_every - step % log_every);
-            DN_TRY(run_small(e, stretch));
-            step += stretch - 1;
-        } else {
+            DN_TRY(run_small(e, stretch, &made));
+            small = made == stretch;  // refused: the kernels of the large path do it
+        }
+        if (made == 0) {
             DN_TRY(step_w(e));
             DN_TRY(step_h(e));
+            made = 1;
         }
+        step += made - 1;
         // "step N: <loss> [<ms> ms/step]" every log_every steps, loss time
         // excluded from the rate (multi_mu_dense_factors_nmf1.h:187-201).
         if (log_every > 0 && (step + 1) % log_every == 0) {

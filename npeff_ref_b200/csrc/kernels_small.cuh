@@ -754,21 +754,32 @@ inline bool small_pays(int64_t nnz, int64_t rows, int r4, int ld) {
     return contract < 60.0 && 20.0 + gather + contract < (ld <= 32 ? 230.0 : (ld <= 64 ? 160.0 : 130.0));
 }
 
+// All blocks have to be on the GPU together: where the process may not use that many SMs (a share of an MPS
+// server, for one) the runtime refuses the launch, and *made says so; nothing has run then.
+// refuse: as if it had.
 template <int LD>
-inline int small_launch_t(SmallArgs& a, cudaStream_t st) {
+inline int small_launch_t(SmallArgs& a, cudaStream_t st, bool refuse, bool* made) {
     DN_CUDA(cudaFuncSetAttribute(k_small_run<LD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem_bytes(LD)));
     void* args[] = {&a};
-    DN_CUDA(cudaLaunchCooperativeKernel((void*)k_small_run<LD>, dim3(kNumSMs), dim3(small_threads(LD)), args, small_smem_bytes(LD), st));
+    const cudaError_t e = refuse ? cudaErrorCooperativeLaunchTooLarge
+                                 : cudaLaunchCooperativeKernel((void*)k_small_run<LD>, dim3(kNumSMs), dim3(small_threads(LD)), args,
+                                                               small_smem_bytes(LD), st);
+    *made = e != cudaErrorCooperativeLaunchTooLarge;
+    if (!*made) {
+        cudaGetLastError();
+        return DNPEFF_OK;
+    }
+    DN_CUDA(e);
     DN_COUNT_LAUNCH(1);
     return DNPEFF_OK;
 }
-inline int small_launch(SmallArgs& a, int ld, cudaStream_t st) {
+inline int small_launch(SmallArgs& a, int ld, cudaStream_t st, bool refuse, bool* made) {
     DN_CUDA(cudaMemsetAsync(a.barrier, 0, 2 * sizeof(unsigned int), st));
     switch (ld) {
-        case 32: return small_launch_t<32>(a, st);
-        case 64: return small_launch_t<64>(a, st);
-        case 96: return small_launch_t<96>(a, st);
-        default: return small_launch_t<128>(a, st);
+        case 32: return small_launch_t<32>(a, st, refuse, made);
+        case 64: return small_launch_t<64>(a, st, refuse, made);
+        case 96: return small_launch_t<96>(a, st, refuse, made);
+        default: return small_launch_t<128>(a, st, refuse, made);
     }
 }
 

@@ -356,6 +356,33 @@ def test_small_problem_barrier_wait_runs_out(torch_cuda):
         assert np.array_equal(eng.load_w_to_host(), want)
 
 
+@pytest.mark.parametrize("iters,log_every", [(7, 0), (5, 2)])
+def test_small_problem_without_room_for_its_launch(torch_cuda, capfd, iters, log_every):
+    """Where the runtime refuses the cooperative launch of the small-problem kernel (the process may use
+    only some of the SMs), the run is made by the large path: the same bits as step by step, and
+    every log line is there."""
+    from npeff_ref_b200 import MuNmfParams
+    n, m, k, r = 200, 4000, 120, 32
+    vals, idx, norms = make_problem(n, m, k, seed=9)
+    with _engine(MuNmfParams(rank=r, eps=1e-8, seed=2, init_scale=0.1), [("refuse_cooperative", 1)]) as eng:
+        eng.set_csr(n, m, vals, idx, None, k, norms, 1)
+        eng.init_factors()
+        for _ in range(iters):
+            eng.step_w()
+            eng.step_h()
+        want = eng.load_w_to_host(), eng.load_h_to_host()
+        eng.init_factors()
+        eng.run(iters, log_every=log_every)
+        got = eng.load_w_to_host(), eng.load_h_to_host()
+        eng.set_option("refuse_cooperative", 0)
+        eng.init_factors()
+        eng.run(iters, log_every=0)
+        small = eng.load_w_to_host()
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+    assert rel_fro(small, want[0]) < 1e-5
+    assert capfd.readouterr().out.count("step ") == (iters // log_every if log_every else 0)
+
+
 # ---------------------------------------------------------------------------
 def test_one_engine_loaded_again_with_other_sizes(torch_cuda):
     """One engine takes matrices of growing and shrinking size (its memory comes from slabs that
