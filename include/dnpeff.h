@@ -17,7 +17,11 @@
  *     one engine per device (one process or thread each) joined by
  *     dnpeff_comm_init; calls on one engine must be serialised by the caller;
  *   - host buffers are caller-owned; device memory is engine-owned and is
- *     released by dnpeff_destroy;
+ *     released by dnpeff_destroy (option keep_memory: up to 8 GB of it a device stay
+ *     for the next engine until dnpeff_release_memory).  What else outlives the
+ *     engines of a process: up to 8 idle streams and 32 MB of page-locked host memory
+ *     (dnpeff_release_memory returns them), 256 KB of page-locked host memory, and
+ *     the scratch of the single-kernel entry points;
  *   - W is [n_rows, rank] row-major, H is [rank, n_cols] row-major at this
  *     boundary: the layouts of the output file (src/io/nmf_decomp_h5.h:38-89);
  *   - values are fp32, column ids int32, row offsets int64.
@@ -80,6 +84,10 @@ int dnpeff_device_count(int* count);
  * `stream` is a cudaStream_t the engine launches on, or NULL to create one. */
 int dnpeff_create(const dnpeff_params* params, int device, void* stream, dnpeff_engine** out);
 int dnpeff_destroy(dnpeff_engine* eng);
+/* Gives back what engines that were destroyed left on `device` (-1: on every one) for
+ * the next, and the idle streams and page-locked chunks of the process.  Engines that
+ * are alive keep what they have.  No reference counterpart (one job per process). */
+int dnpeff_release_memory(int device);
 
 /* Engine options: tuning values and test hooks (no reference counterpart; the
  * reference has no tunables beyond MuNmfParams).  Set before the call they affect;
@@ -100,6 +108,14 @@ int dnpeff_destroy(dnpeff_engine* eng);
  *                       between the blocks of the small-problem kernel,
  *                       gives up (default 2^24); the kernel then leaves cleanly and the
  *                       next call that reads the engine's status returns DNPEFF_ERR_CUDA
+ *   "keep_memory"       1: dnpeff_destroy leaves the engine's device memory, up to 8 GB a
+ *                       device with what lies there already, for the next engine of
+ *                       the process: for programs that run one job after the other
+ *                       (allocating and freeing is a quarter of a small one's time).  It
+ *                       goes back to the device when an allocation of this library
+ *                       fails, when an engine with this option ends that never needed
+ *                       it, and with dnpeff_release_memory; no other allocator can
+ *                       have it before (default 0)
  *   "refuse_cooperative" 1: the launch of the small-problem kernel, whose blocks must all
  *                       be on the GPU together, is treated as refused, as the runtime
  *                       does where the process may use only some of the SMs (test hook);

@@ -6,4 +6,4 @@ mirrors the reference's ``MuNmf`` interface.  There is no CPU fallback: if the
 library is missing or no CUDA device answers, calls raise.
 """
 from ._lib import DnpeffError, lib, lib_path  # noqa: F401
-from .engine import MuNmf, MuNmfParams, preprocess_and_split  # noqa: F401
+from .engine import MuNmf, MuNmfParams, preprocess_and_split, release_memory  # noqa: F401

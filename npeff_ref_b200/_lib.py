@@ -36,6 +36,7 @@ SIGNATURES = {
     "dnpeff_device_count": (C.c_int, [C.POINTER(C.c_int)]),
     "dnpeff_create": (C.c_int, [C.POINTER(Params), C.c_int, _P, C.POINTER(_P)]),
     "dnpeff_destroy": (C.c_int, [_P]),
+    "dnpeff_release_memory": (C.c_int, [C.c_int]),
     "dnpeff_set_option": (C.c_int, [_P, C.c_char_p, _I64]),
     "dnpeff_set_csr": (C.c_int, [_P, _I64, _I64, _I64, _P, _P, _P, _P, _I32]),
     "dnpeff_row_slice": (C.c_int, [_I64, _I32, _I32, C.POINTER(_I64), C.POINTER(_I64)]),

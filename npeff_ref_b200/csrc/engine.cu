@@ -160,6 +160,7 @@ struct dnpeff_engine {
     uint32_t opt_wait_limit = kTiledSpinLimit;
     bool opt_keep_csr = false;
     bool opt_refuse_cooperative = false;
+    bool opt_keep_memory = false;
 };
 
 namespace {
@@ -1512,12 +1513,22 @@ int dnpeff_destroy(dnpeff_engine* e) {
     cudaStreamSynchronize(e->st);
     if (e->comm) nccl_api().CommDestroy(e->comm);
     if (e->up) StreamCache::get().give(e->device, e->up);
-    e->arena.close();
+    e->arena.close(e->opt_keep_memory);
     PinnedSlots::get().give(e->h_pinned);
     for (auto& r : e->regions) { cudaEventDestroy(r.a); cudaEventDestroy(r.b); }
     for (auto ev : e->ev_pool) cudaEventDestroy(ev);
     if (e->own_stream) StreamCache::get().give(e->device, e->st);
     delete e;
+    return DNPEFF_OK;
+}
+
+int dnpeff_release_memory(int device) {
+    int ndev = 0;
+    DN_CUDA(cudaGetDeviceCount(&ndev));
+    if (device < -1 || device >= ndev) return fail(DNPEFF_ERR_INVALID, "device %d of %d", device, ndev);
+    SlabCache::get().flush(device);
+    StreamCache::get().flush(device);
+    StagingRing::get().release();
     return DNPEFF_OK;
 }
 
@@ -1534,6 +1545,8 @@ int dnpeff_set_option(dnpeff_engine* e, const char* name, int64_t value) {
         e->opt_popular_divisor = (int)value;
     } else if (!strcmp(name, "keep_canonical_csr")) {
         e->opt_keep_csr = value != 0;
+    } else if (!strcmp(name, "keep_memory")) {
+        e->opt_keep_memory = value != 0;
     } else if (!strcmp(name, "refuse_cooperative")) {
         e->opt_refuse_cooperative = value != 0;
     } else if (!strcmp(name, "wait_limit")) {

@@ -10,11 +10,11 @@
 
 namespace dnpeff {
 
-// Slabs left behind by engines that were destroyed, for the next engine on the same device: a
-// program that factorizes one small matrix after another would otherwise spend more time in
-// cudaMalloc and cudaFree than in its kernels, and one with data sets of half a gigabyte (4 GB of slabs each) 9 of
-// 75 ms.  At most kMost bytes a device, a twentieth of its memory; they go back to the device when an allocation fails, and when an engine ends
-// that never needed them.
+// Slabs that engines left when they were destroyed (those that were asked to, option keep_memory), for
+// the next engine on the same device: whole jobs from host memory, 300 x 9000 at rank 128 and 8192 x 1048576
+// at rank 64 (4 GB of slabs each), take 6.8 and 77 ms without and 5.1 and 63 with it, the
+// rest being cudaMalloc and cudaFree.  At most kMost bytes a device, a twentieth of its memory; they go back to the
+// device when an allocation here fails, when an engine ends that never needed them, and with dnpeff_release_memory.
 class SlabCache {
 public:
     static constexpr size_t kMost = (size_t)8 << 30;
@@ -60,10 +60,10 @@ public:
             }
         }
     }
-    void flush(int device) {
+    void flush(int device) {  // (-1: of every device)
         std::lock_guard<std::mutex> lk(mu_);
         for (auto it = slabs_.begin(); it != slabs_.end();) {
-            if (it->device == device) {
+            if (device < 0 || it->device == device) {
                 cudaFree(it->p);
                 it = slabs_.erase(it);
             } else {
@@ -107,6 +107,17 @@ public:
                 }
         }
         return cudaStreamCreateWithFlags(out, cudaStreamNonBlocking);
+    }
+    void flush(int device) {  // (-1: of every device)
+        std::lock_guard<std::mutex> lk(mu_);
+        for (auto it = idle_.begin(); it != idle_.end();) {
+            if (device < 0 || it->first == device) {
+                cudaStreamDestroy(it->second);
+                it = idle_.erase(it);
+            } else {
+                ++it;
+            }
+        }
     }
     void give(int device, cudaStream_t st) {
         if (cudaStreamSynchronize(st) == cudaSuccess) {
@@ -251,11 +262,15 @@ public:
         }
     }
 
-    // Everything goes, live or not (the engine is being destroyed, its streams are idle).
-    void close() {
+    // Everything goes, live or not (the engine is being destroyed, its streams are idle): to the next engine
+    // (keep) or to the device.
+    void close(bool keep) {
         std::vector<std::pair<char*, size_t>> all;
-        for (auto& kv : slabs_) all.push_back({kv.first, kv.second.bytes});
-        SlabCache::get().give(device_, std::move(all), born_);
+        for (auto& kv : slabs_) {
+            if (keep) all.push_back({kv.first, kv.second.bytes});
+            else cudaFree(kv.first);
+        }
+        if (keep) SlabCache::get().give(device_, std::move(all), born_);
         slabs_.clear();
         live_.clear();
     }

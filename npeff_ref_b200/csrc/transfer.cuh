@@ -30,7 +30,7 @@ inline bool host_pageable(const void* p) {
 }
 
 // The process's page-locked chunks: kThreads threads, two chunks each (32 MB, made on first use
-// and kept: page-locking them takes as long as moving several hundred MB).  One transfer at a
+// and kept until dnpeff_release_memory: page-locking them takes as long as moving several hundred MB).  One transfer at a
 // time holds them; whoever finds them taken copies the plain way.
 struct StagingRing {
     static constexpr int kThreads = 8;
@@ -48,6 +48,12 @@ struct StagingRing {
             base = nullptr;
         }
         return base != nullptr;
+    }
+    void release() {  // unless a transfer holds them
+        std::unique_lock<std::mutex> lk(mu, std::try_to_lock);
+        if (!lk.owns_lock() || !base) return;
+        cudaFreeHost(base);
+        base = nullptr;
     }
     // Threads worth starting for that many bytes (starting one costs about what it takes to copy
     // a quarter of a megabyte), and the bytes that one handles at a time.

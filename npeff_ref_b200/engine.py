@@ -34,16 +34,26 @@ def _ptr(a):
     return None if a is None else C.c_void_p(a.ctypes.data)
 
 
+def release_memory(device=-1):
+    """Device memory that closed engines left for the next one (``MuNmf(keep_memory=True)``), of one
+    device or of all, goes back to it; so do the process's idle streams and page-locked chunks."""
+    check(lib().dnpeff_release_memory(int(device)))
+
+
 class MuNmf:
+    """One shard on one device.  ``keep_memory``: :meth:`close` leaves the device memory, at most 8 GB a
+    device, to the next engine of the process until :func:`release_memory`; without it, close gives
+    everything back at once, as ``dnpeff_destroy`` does by default."""
     CONTIGUOUS, CYCLIC = 0, 1
 
-    def __init__(self, params, device=0, shard_index=0, n_shards=1, stream=None, shard_mode=0):
+    def __init__(self, params, device=0, shard_index=0, n_shards=1, stream=None, shard_mode=0, keep_memory=True):
         self.params = params
         self._h = C.c_void_p()
         p = Params(int(params.rank), float(params.eps), int(params.seed),
                    float(params.init_scale), int(shard_index), int(n_shards), int(shard_mode))
         check(lib().dnpeff_create(C.byref(p), int(device), C.c_void_p(stream or 0),
                                   C.byref(self._h)))
+        self.set_option("keep_memory", bool(keep_memory))
         self.device = device
         self.shard_index = shard_index
         self.n_shards = n_shards

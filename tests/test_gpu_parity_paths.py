@@ -383,6 +383,47 @@ def test_small_problem_without_room_for_its_launch(torch_cuda, capfd, iters, log
     assert capfd.readouterr().out.count("step ") == (iters // log_every if log_every else 0)
 
 
+@pytest.mark.parametrize("keep", [False, True])
+def test_device_memory_after_destroy(torch_cuda, keep):
+    """dnpeff_destroy gives the device memory back; with keep_memory it stays for the next engine, which
+    uses it, and dnpeff_release_memory gives it back.  Free memory as the device reports it, to 32 MB
+    (modules that load on first use are loaded by a first engine)."""
+    from npeff_ref_b200 import MuNmfParams, release_memory
+    torch = torch_cuda
+    n, m, k, r = 64, 1 << 20, 8, 128
+    rng = np.random.default_rng(0)
+    idx = np.stack([rng.choice(m, k, replace=False) for _ in range(n)]).astype(np.int32)
+    vals = rng.random((n, k), dtype=np.float32)
+
+    def free():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    def job(keep):
+        # a list of kept columns makes H large with few entries: 524288 x 128 floats
+        eng = _engine(MuNmfParams(rank=r, eps=1e-8), keep_memory=keep)
+        eng.set_csr_retain(n, m, vals, idx, np.arange(1 << 19, dtype=np.int32), None, k)
+        eng.init_factors()
+        eng.step_w()
+        eng.step_h()
+        inside = free()
+        eng.close()
+        return inside
+
+    job(False)
+    release_memory()
+    before = free()
+    inside = job(keep)
+    after = free()
+    assert before - inside > (400 << 20)       # H and A^T W, 256 MB each
+    if keep:
+        assert before - after > (400 << 20)
+        assert abs(job(True) - inside) < (32 << 20)
+        release_memory(0)
+        after = free()
+    assert before - after < (32 << 20)
+
+
 # ---------------------------------------------------------------------------
 def test_one_engine_loaded_again_with_other_sizes(torch_cuda):
     """One engine takes matrices of growing and shrinking size (its memory comes from slabs that
