@@ -657,9 +657,8 @@ int load_device(dnpeff_engine* e, int64_t n, int64_t m_full, int64_t k, const in
     if (pad_bytes > kSmallBytes && e->p.n_shards == 1) {  // (the engines of a job must agree on the stride)
         // the factors and the products of their shape (three of each side) must not take a
         // quarter of the free memory more than without the padding
-        size_t free_b = 0, total_b = 0;
-        DN_CUDA(cudaMemGetInfo(&free_b, &total_b));
-        free_b += e->arena.unused();
+        size_t free_b = 0;
+        DN_TRY(e->arena.at_hand(&free_b));
         if (pad_bytes > 0.25 * (double)free_b) ld = r;
     }
     e->ld = ld;
@@ -708,9 +707,8 @@ int load_device(dnpeff_engine* e, int64_t n, int64_t m_full, int64_t k, const in
     if (dense && 8.0 * (double)n * (double)n_hot > kSmallBytes) {
         // both dense copies (8 bytes per element of the block) within a third of
         // the memory that is free now
-        size_t free_b = 0, total_b = 0;
-        DN_CUDA(cudaMemGetInfo(&free_b, &total_b));
-        free_b += e->arena.unused();
+        size_t free_b = 0;
+        DN_TRY(e->arena.at_hand(&free_b));
         max_hot = (int64_t)(free_b / 3 / (8 * (size_t)std::max<int64_t>(n, 1)));
         max_hot = std::min<int64_t>(max_hot / 128 * 128, (int64_t)1 << 21);
         if (max_hot < 128) {

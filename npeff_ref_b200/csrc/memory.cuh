@@ -71,6 +71,13 @@ public:
             }
         }
     }
+    size_t held(int device) {
+        std::lock_guard<std::mutex> lk(mu_);
+        size_t n = 0;
+        for (auto& s : slabs_)
+            if (s.device == device) n += s.bytes;
+        return n;
+    }
     int64_t now() {
         std::lock_guard<std::mutex> lk(mu_);
         return ++clock_;
@@ -208,7 +215,8 @@ public:
         const size_t take = own ? best_len : bytes;
         if (best_len > take) s.free[best_off + take] = best_len - take;
         s.used += take;
-        live_[best->first + best_off] = take;
+        live_[best->first + best_off] = {take, bytes};
+        asked_ += bytes;
         *out = best->first + best_off;
         return DNPEFF_OK;
     }
@@ -216,7 +224,8 @@ public:
     void release(void* p) {
         auto it = live_.find((char*)p);
         if (it == live_.end()) return;
-        size_t len = it->second;
+        size_t len = it->second.first;
+        asked_ -= it->second.second;
         live_.erase(it);
         auto sl = std::prev(slabs_.upper_bound((char*)p));
         Slab& s = sl->second;
@@ -237,12 +246,29 @@ public:
         s.free[off] = len;
     }
 
-    // Bytes of slabs without a live block: free memory, to whoever asks the device.
+    // Bytes of slabs without a live block.
     size_t unused() const {
         size_t n = 0;
         for (auto& kv : slabs_)
             if (kv.second.used == 0) n += kv.second.bytes;
         return n;
+    }
+
+    // Memory that the engine may plan with: what the device has free, and what lies in the engine's slabs and in
+    // those that other engines left beyond what live blocks asked for.  The same for the same load whatever
+    // slabs there are from earlier ones, so that sizes derived from it (and with them the order of sums) do not
+    // depend on a process's history.  What others hold counts; to five leading bits, so
+    // that a module loaded meanwhile hardly ever does.
+    int at_hand(size_t* out) const {
+        size_t free_b = 0, total_b = 0;
+        DN_CUDA(cudaMemGetInfo(&free_b, &total_b));
+        for (auto& kv : slabs_) free_b += kv.second.bytes;
+        free_b += SlabCache::get().held(device_);
+        free_b -= std::min(free_b, asked_);
+        size_t unit = 1;
+        while (free_b / unit >= 32) unit *= 2;
+        *out = free_b / unit * unit;
+        return DNPEFF_OK;
     }
 
     // Slabs without a live block go back to the device until at most `keep` unused bytes are left.
@@ -273,6 +299,7 @@ public:
         if (keep) SlabCache::get().give(device_, std::move(all), born_);
         slabs_.clear();
         live_.clear();
+        asked_ = 0;
     }
 
 private:
@@ -282,7 +309,8 @@ private:
         std::map<size_t, size_t> free;  // offset -> length
     };
     std::map<char*, Slab> slabs_;
-    std::map<char*, size_t> live_;
+    std::map<char*, std::pair<size_t, size_t>> live_;  // length, and what was asked for
+    size_t asked_ = 0;
     cudaStream_t st_ = nullptr;
     int device_ = 0;
     int64_t born_ = 0;

@@ -424,6 +424,52 @@ def test_device_memory_after_destroy(torch_cuda, keep):
     assert before - after < (32 << 20)
 
 
+def test_layout_near_the_memory_cap_does_not_depend_on_earlier_engines(torch_cuda):
+    """Where the dense block is capped by the free memory, what earlier engines left for the next one, and
+    what the engine itself holds from an earlier load, counts as free: the same popular columns and the same
+    bits of W from a fresh process's engine, from one that comes after others, and from one loaded again."""
+    from npeff_ref_b200 import MuNmfParams, release_memory
+    from npeff_ref_b200._lib import lib, check
+    torch = torch_cuda
+    n, m, k, r = 8192, 40000, 2048, 32
+    vals = torch.empty((n, k), dtype=torch.float32, device="cuda")
+    idx = torch.empty((n, k), dtype=torch.int32, device="cuda")
+    norms = torch.empty(n, dtype=torch.float32, device="cuda")
+    check(lib().dnpeff_synth_pef_device(n, m, k, 0.05, 1.0, 3, vals.data_ptr(), idx.data_ptr(), norms.data_ptr(),
+                                        torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+
+    def load(eng):
+        eng.set_csr_device(n, m, vals.data_ptr(), idx.data_ptr(), 0, k, norms.data_ptr(), 1)
+        eng.init_factors()
+        eng.step_w()
+        eng.step_h()
+        eng.step_w()
+        return eng.layout()[0], eng.load_w_to_host()
+
+    params = MuNmfParams(rank=r, eps=1e-8, seed=1, init_scale=0.1)
+    with _engine(params) as eng:               # modules that load on first use
+        load(eng)
+    release_memory()
+    torch.cuda.empty_cache()
+    filler = torch.empty(torch.cuda.mem_get_info()[0] - (11 << 29), dtype=torch.uint8, device="cuda")  # 5.5 GB are left
+    try:
+        with _engine(params) as eng:
+            first = load(eng)
+            again = load(eng)
+        with _engine(MuNmfParams(rank=128, eps=1e-8, seed=1, init_scale=0.1)) as eng:
+            load(eng)                          # leaves slabs of other sizes
+        with _engine(params) as eng:
+            later = load(eng)
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+        release_memory()
+    assert 128 <= first[0] < 30000             # capped: 40000 columns are held by a 32nd of the rows
+    for got in (again, later):
+        assert got[0] == first[0] and np.array_equal(got[1], first[1])
+
+
 # ---------------------------------------------------------------------------
 def test_one_engine_loaded_again_with_other_sizes(torch_cuda):
     """One engine takes matrices of growing and shrinking size (its memory comes from slabs that
