@@ -182,6 +182,10 @@ constexpr int kMaxHotTiles = 1024;            // tiles of popular columns per ro
 // every further launch costs about 11 us: 48 MB is the measured optimum on B200.
 constexpr int64_t kTailBlockBytes = 48 << 20;
 constexpr int kMaxTailBlocks = 512;
+// Most that padding the rank may add to an engine of a sharded job: an eighth of the GPU's 180 GB.  The
+// allreduce of A*H^T grows with the stride too, and is not bounded: by arithmetic 1.4 ns a row at rank 130 as 256 (504
+// more bytes at 725 GB/s, twice), about what the CUDA cores take for the contractions of a row of W.
+constexpr double kShardedPadBytes = 22.5e9;
 constexpr int kSmallIters = 256;              // iterations per launch of the small-problem kernel
 constexpr int kFitSteps = 256;                // W-only steps per launch (a tile's step takes 5 to 40 us)
 
@@ -653,10 +657,15 @@ int load_device(dnpeff_engine* e, int64_t n, int64_t m_full, int64_t k, const in
     int ld = padded_rank(r, e->p.eps);
     // Asking the device for its free memory takes 0.1 ms or more: not for small matrices.
     constexpr double kSmallBytes = 256 << 20;
-    const double pad_bytes = (double)(ld - r) * 12.0 * (double)(n + ms);
-    if (pad_bytes > kSmallBytes && e->p.n_shards == 1) {  // (the engines of a job must agree on the stride)
-        // the factors and the products of their shape (three of each side) must not take a
-        // quarter of the free memory more than without the padding
+    // Three arrays of either side's shape: the factors and the products of theirs.
+    const int64_t ms_most = m_kept / e->p.n_shards + e->p.n_shards;  // of any shard
+    const double pad_bytes = (double)(ld - r) * 12.0 * (double)(n + (e->p.n_shards > 1 ? ms_most : ms));
+    if (e->p.n_shards > 1) {
+        // The engines of a job must agree on the stride without asking one another: by sizes that
+        // all of them know.
+        if (pad_bytes > kShardedPadBytes) ld = r;
+    } else if (pad_bytes > kSmallBytes) {
+        // not a quarter of the free memory more than without the padding
         size_t free_b = 0;
         DN_TRY(e->arena.at_hand(&free_b));
         if (pad_bytes > 0.25 * (double)free_b) ld = r;

@@ -470,6 +470,26 @@ def test_layout_near_the_memory_cap_does_not_depend_on_earlier_engines(torch_cud
         assert got[0] == first[0] and np.array_equal(got[1], first[1])
 
 
+@pytest.mark.parametrize("n_shards,m_kept,padded", [(2, 1 << 20, True), (2, 31_000_000, False), (1, 1 << 20, True)])
+def test_padding_of_a_sharded_rank_is_bounded(torch_cuda, n_shards, m_kept, padded):
+    """Rank 130 is stored with a stride of 256 while that costs an engine of a job at most 22.5 GB, by sizes
+    that all engines know, and as it is beyond.  The stride shows in the memory that H takes."""
+    from npeff_ref_b200 import MuNmfParams, release_memory
+    n, k, r = 40, 4, 130
+    rng = np.random.default_rng(1)
+    idx = np.stack([rng.choice(m_kept, k, replace=False) for _ in range(n)]).astype(np.int32)
+    vals = rng.random((n, k), dtype=np.float32)
+    free = torch_cuda.cuda.mem_get_info
+    with _engine(MuNmfParams(rank=r), keep_memory=False, n_shards=n_shards) as eng:
+        release_memory()
+        before = free()[0]
+        eng.set_csr_retain(n, m_kept, vals, idx, np.arange(m_kept, dtype=np.int32), None, k)
+        columns = eng.shape[3]
+        used = before - free()[0]
+    assert columns == m_kept // n_shards
+    assert (used > 4 * columns * 220) == padded      # H: 520 bytes a column, or 1024
+
+
 # ---------------------------------------------------------------------------
 def test_one_engine_loaded_again_with_other_sizes(torch_cuda):
     """One engine takes matrices of growing and shrinking size (its memory comes from slabs that
