@@ -272,7 +272,9 @@ int padded_rank(int r, float eps) {
 
 // Popular columns hold at least ceil(n / div) entries.  In the dense tensor-core block a column of 20000
 // rows costs 16 ns a product whatever it holds (rank 128), its entries 31 ps each in the sparse one: even at
-// a 37th stored, and flat around it (configuration 2, ms per iteration: 24.3 at 16, 23.1 at 32, 23.3 at 40).
+// a 37th stored, and flat around it (ms per iteration at 16, 32, 48 and 64, configuration 2: 24.3, 22.7, 22.7, 23.4;
+// a sixteenth of configuration 3, rank 256: -, 13.1, 13.1, 13.6; of 5, rank 512: -, 17.0, 17.0, 17.5; 5003 x 300007 at
+// rank 100: -, 0.97, 0.98, 1.00).
 // With few rows much of the block is the padding of its last tile.  The sparse tiled kernel needs longer columns.
 int hot_divisor(const dnpeff_engine* e, bool dense, int64_t n) {
     if (e->opt_popular_divisor >= 2) return e->opt_popular_divisor;
@@ -299,9 +301,15 @@ size_t gram_any_scratch(int64_t rows, int r) {
     return a > b ? a : b;
 }
 
-// Several steps on the CUDA cores or on the tensor cores (us per step, 2000 and 10000 rows): rank 32 0.33, 1.1 | 6.0;
-// 64 0.76, 3.7 | 8.3; 96 1.8, 8.2 | 10.0; 128 2.6, 11.6 | 10.7, where the lines cross at 9000 rows.
-bool fit_on_cuda_cores(int64_t rows, int r) { return r < 128 || rows <= 9000; }
+// Several steps on the CUDA cores, whose time grows with the rows, or on the tensor cores, whose time grows by
+// waves of 148 tiles of 128 rows.  us per step at 2000, 10000 and 18944 rows | a full wave: rank 32 0.33, 1.1, 1.4 | 6.0;
+// 64 0.76, 3.7, 6.0 | 8.1; 96 1.9, 8.3, 14.8 | 10.1; 128 2.6, 11.6, - | 10.7.  So 32 and 64 stay on the CUDA cores; the
+// lines cross at 9000 rows at 128, and at 96 at 12000 rows a wave (12000: 10.1 either way; 18945: 15.6 against 18.1;
+// 25000: 20.2 against 20.0; 37888: 29.6 against 20.1; 37889: 30.2 against 27.8; 50000: 39.4 against 30.1).
+bool fit_on_cuda_cores(int64_t rows, int r) {
+    const int64_t waves = ceil_div(rows, (int64_t)kNumSMs * 128);
+    return r < 96 || rows <= (r == 96 ? 12000 * waves : 9000);
+}
 
 // `steps` updates of X.  gsplit: 2*r*r floats that hold the split G already (have_split) or are
 // scratch for it.

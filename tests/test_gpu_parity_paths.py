@@ -587,6 +587,13 @@ def test_w_only_steps_match_single_steps(torch_cuda, n, r):
         assert rel_fro(eng.load_w_to_host(), want) < 1e-5
 
 
+@pytest.mark.parametrize("n,r", [(12000, 96), (12001, 96), (18944, 90), (18945, 96), (24001, 96)])
+def test_w_only_steps_where_rank_96_changes_kernels(torch_cuda, n, r):
+    """Rank 96 leaves the CUDA cores at 12000 rows a wave of the tensor-core kernel: either side of it, the
+    last row of the first wave and the first of the second (the bound of the test above)."""
+    test_w_only_steps_match_single_steps(torch_cuda, n, r)
+
+
 @pytest.mark.parametrize("r", [64, 100, 128])
 def test_large_h_into_page_locked_memory(torch_cuda, r):
     """A large H read back in parts (page-locked destination) against the one copy into pageable memory; 100: a ragged last part."""
