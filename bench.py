@@ -43,16 +43,10 @@ EPS = 1e-12
 METRIC = "dnpeff_nmf_iterations_per_s"
 UNIT = "iter/s"
 
-# dram__bytes_read.sum + dram__bytes_write.sum of one A*H^T product (a sequence of
-# launches: the dense popular block on tensor cores + one launch per tail column
-# block), keyed by (config, ranks, product).  Config 2 on one GPU: scaled from an ncu
-# capture of the same workload with a tenth of the rows, where the product moved
-# 3.06 GB: 2.01 GB are the dense factor H, read once whatever the row count; the
-# other 1.05 GB (dense block of A, tail entries, split-K partials) grow with the
-# rows: 2.15e9 (H at full size) + 10 * 1.05e9.
-# (12.6 GB with the popular columns of that capture; the 67 929 columns that are dense since then add
-# 20000 x 4 bytes each and take 59 M entries of 8 bytes out of the tail)
-NCU_TRAFFIC_BYTES = {(2, 1, "spmm_ah"): 12.6e9 + 67929 * 20000 * 4 - 59.0e6 * 8}
+# dram__bytes_read.sum + dram__bytes_write.sum of one sparse product (a sequence of launches: the dense
+# popular block on tensor cores, then the tail), keyed by (config, ranks, product).  Config 2 on one GPU: both
+# products captured whole at this size (profiles/spmm_products_config2_dram_bytes.md), 17.0 + 0.3 GB and 14.5 + 2.3 GB.
+NCU_TRAFFIC_BYTES = {(2, 1, "spmm_ah"): 17.34e9, (2, 1, "spmm_wa"): 16.81e9}
 
 
 def workload_name(cfg_id, c):
@@ -509,7 +503,7 @@ def main():
                       "what": "tail entries x 4r bytes / product time, against 148 SMs x 64 B/clk at the sampled SM clock"},
         "note": "one product = the dense popular block on tensor cores + one launch per tail column block, timed as a whole; "
                 "every stored entry gathers r floats on chip (shared memory or L2), so the SpMM is not "
-                "HBM-bound for r >= 64; traffic is scaled from a small-case capture",
+                "HBM-bound for r >= 64; traffic was captured at this size (dram bytes read and written), not in this run",
     }
     # the loss after exactly K iterations from the seeded initial factors: what the
     # end-to-end run below must arrive at (untimed)
