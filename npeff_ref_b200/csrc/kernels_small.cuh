@@ -4,12 +4,18 @@
 // the kernels of the large path -- fourteen launches per iteration, each with a pipeline of
 // copies, tensor-core runs and drains to fill and empty -- take 100 to 150 us for it whatever its
 // size.  Here one cooperative launch makes many iterations: a persistent block per SM, everything
-// L2-resident, CUDA-core arithmetic, four grid-wide barriers per iteration:
+// L2-resident, the contractions on the CUDA cores (strides 32 and 64) or on mma.sync fragments (96 and
+// 128), four grid-wide barriers per iteration:
 //
 //   A  numerators of W: A * H^T, flat over the stored entries | H H^T from the blocks' partials
 //   B  W *= num / (W HH + eps), row tiles; each block's partial of W^T W on the way
 //   C  numerators of H: A^T * W                               | W^T W from the partials
 //   D  H *= num / (H WW + eps); each block's partial of H H^T
+//
+// us per iteration of A's and C's products, their Gram sums, B and D, each with its barrier (block 0's clock):
+// 64 x 1612, stride 32, 6144 entries: 2.7, 2.7, 2.1, 7.2, 7.4; 2048 x 65536, 32, 8.4 M: 72, 73, 2.4, 8.7, 22 (14.9 TB/s
+// of gathered rows); 1777 x 43231, 32 (rank 20), 0.83 M: 9.7, 10.7, 2.1, 7.7, 17.6; 300 x 9000, 128, 0.45 M: 19.3, 19.2,
+// 6.3, 9.2, 21.1 (11.9 TB/s).
 //
 // Sparse products.  The stored entries are cut into units of L consecutive entries, one per lane
 // group (LD / 4 lanes, a float4 of the factor row each); a unit adds up its entries row by row.
@@ -742,8 +748,8 @@ inline int small_tile_rows(int64_t rows, int ld) {
 }
 
 // Whether these launches beat the large path.  An iteration takes about 20 us (barriers, and the
-// latency of the four phases), two gathers of a factor row per stored entry at the L2 ports' rate
-// and the two contractions at what shared memory delivers to the CUDA cores.  The large path
+// latency of the four phases), two gathers of a factor row per stored entry at 15 TB/s (12 at the wide strides;
+// measured: 14.9 and 11.9) and the two contractions at what shared memory delivers to the cores.  The large path
 // takes 65 to 105 us plus the same gathers a little slower, but contracts on the tensor cores: even near
 // 230 us in all at stride 32 (3000 x 60000 x 4000 values: 233 either way; half of them 136 against 175),
 // 160 at 64 (2000 x 40000 x 2000: 182 against 167; 500 x 20000 x 2000: 75 against 109) and 130 above
