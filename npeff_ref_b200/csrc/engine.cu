@@ -111,7 +111,7 @@ struct dnpeff_engine {
     BlockTcPlan plan_x1 = {}, plan_x2 = {};
     uint32_t* x1_max = nullptr;  // bits of the largest magnitude per row of x1; then
     uint32_t* x2_max = nullptr;  // per row of x2, and
-    uint32_t* y_max[2] = {nullptr, nullptr};  // per column of the factor, of products in turn (ld words each)
+    uint32_t* y_max[2] = {nullptr, nullptr};  // per column of the factor, of products in turn (ld words each), then
     unsigned long long* x1_sum = nullptr;     // sums that say where the halves do not do (blk_faint), per row of x1; then
     unsigned long long* x2_sum = nullptr;     // per row of x2, and
     unsigned char* blk_again = nullptr;       // a byte per row of a product
@@ -367,7 +367,7 @@ void free_matrix(dnpeff_engine* e) {
     dev_free(e, e->new_to_og);
     dev_free(e, e->perm); dev_free(e, e->inv_perm);
     dev_free(e, e->b_vals); dev_free(e, e->b_col); dev_free(e, e->tail_off);
-    dev_free(e, e->x1); dev_free(e, e->x2); dev_free(e, e->x1_max); dev_free(e, e->x1_sum); dev_free(e, e->blk_ysplit); dev_free(e, e->blk_partial);
+    dev_free(e, e->x1); dev_free(e, e->x2); dev_free(e, e->x1_max); dev_free(e, e->blk_ysplit); dev_free(e, e->blk_partial);
     e->tail_nnz.clear();
     e->n_hot = 0; e->n_tail_blocks = 0; e->hot_nnz = 0;
     dev_free(e, e->W); dev_free(e, e->H); dev_free(e, e->AHG); dev_free(e, e->WA); dev_free(e, e->WW);
@@ -804,16 +804,15 @@ int load_device(dnpeff_engine* e, int64_t n, int64_t m_full, int64_t k, const in
             DN_TRY(dev_alloc(e, &e->x1, e->plan_x1.x_halves));
             DN_TRY(dev_alloc(e, &e->x2, e->plan_x2.x_halves));
             const size_t maxima = e->plan_x1.xmax_words + e->plan_x2.xmax_words + 2 * (size_t)ld;
-            DN_TRY(dev_alloc(e, &e->x1_max, maxima));
+            const size_t sums = e->plan_x1.xmax_words + e->plan_x2.xmax_words, flags4 = (size_t)(std::max(n, n_hot) + 3) / 4;
+            DN_TRY(dev_alloc(e, &e->x1_max, maxima + 2 * sums + flags4));
             e->x2_max = e->x1_max + e->plan_x1.xmax_words;
             e->y_max[0] = e->x2_max + e->plan_x2.xmax_words;
             e->y_max[1] = e->y_max[0] + ld;
-            DN_CUDA(cudaMemsetAsync(e->x1_max, 0, sizeof(uint32_t) * maxima, st));
-            const size_t sums = e->plan_x1.xmax_words + e->plan_x2.xmax_words, flags8 = (size_t)(std::max(n, n_hot) + 7) / 8;
-            DN_TRY(dev_alloc(e, &e->x1_sum, sums + flags8));
+            e->x1_sum = (unsigned long long*)(e->x1_max + maxima);
             e->x2_sum = e->x1_sum + e->plan_x1.xmax_words;
             e->blk_again = (unsigned char*)(e->x1_sum + sums);
-            DN_CUDA(cudaMemsetAsync(e->x1_sum, 0, sizeof(*e->x1_sum) * (sums + flags8), st));
+            DN_CUDA(cudaMemsetAsync(e->x1_max, 0, sizeof(uint32_t) * (maxima + 2 * sums + flags4), st));
             DN_TRY(dev_alloc(e, &e->blk_ysplit, std::max(e->plan_x1.ysplit_halves, e->plan_x2.ysplit_halves)));
             DN_TRY(dev_alloc(e, &e->blk_partial, std::max(e->plan_x1.partial_floats, e->plan_x2.partial_floats)));
             DN_CUDA(cudaMemsetAsync(e->x1, 0, sizeof(__half) * e->plan_x1.x_halves, st));
