@@ -16,7 +16,7 @@
 // lost: a numerator that comes out zero would hold its factor entry at zero for good.  Rows of X and
 // columns of Y with faint values are marked, and where such a row or column meets a sum so small that the
 // representation could be off by 2^-23 of it, the row of C is computed again from the values themselves
-// (blk_faint, k_block_repair).
+// (blk_faint, blk_repair_row).
 //
 // Layouts.  X is split when the matrix is loaded (4 bytes per element, as fp32), in blocks of 128
 // rows x 64 K-values, block (tile, chunk) at (tile * k_chunks + chunk) * 32 KB: [hi | lo], each in the
@@ -140,6 +140,15 @@ __device__ __forceinline__ uint32_t blk_count_faint(const float (&v)[8], float s
     return n;
 }
 
+// Whether any of them is, under the scale of the maximum's word: the smallest magnitude other than zero (2 * bits - 1
+// drops the sign and makes zero the largest) against the power of two that the scale takes to kBlkFaint.
+__device__ __forceinline__ bool blk_any_faint(const float (&v)[8], uint32_t word) {
+    uint32_t least = 0xffffffffu;
+#pragma unroll
+    for (int t = 0; t < 8; t++) least = min(least, 2u * __float_as_uint(v[t]) - 1u);
+    return least < 2u * __float_as_uint(kBlkFaint * blk_unscale(word)) - 1u;
+}
+
 // The smallest lo half for values other than zero that both halves would lose.
 __device__ __forceinline__ uint32_t blk_lost2(float x, float y, uint32_t hi, uint32_t lo) {
     const uint32_t some = hi | lo;
@@ -197,7 +206,7 @@ __global__ void k_split_y(const float* __restrict__ Y, int64_t K, int r, int pn,
     uint4 hi, lo;
     const uint32_t most = ymax[col];
     blk_split8(v, most, hi, lo);
-    if (blk_count_faint(v, blk_scale(most)) && !(__ldcg(ymax + col) & kBlkMark)) atomicOr(ymax + col, kBlkMark);
+    if (blk_any_faint(v, most) && !(__ldcg(ymax + col) & kBlkMark)) atomicOr(ymax + col, kBlkMark);
     const int64_t c = ko / 8;
     __half* base = Ysplit + (panel * k_chunks + c) * (2 * 64) * pn + blk_canon(n, (int)(ko % 8) * 8);
     *(uint4*)base = hi;
@@ -209,8 +218,10 @@ __device__ __forceinline__ float4 blk_unscaled4(const float4& v, uint32_t row_wo
                        blk_unscaled(v.w, row_word, m.w));
 }
 // Whether one of four sums at `at` wants computing again.
-__device__ __forceinline__ bool blk_again(const float4& v, uint32_t row_word, const uint4& m, float row_sum,
-                                          const float* __restrict__ keep, int64_t at) {
+__device__ __forceinline__ bool blk_again(const float4& v, uint32_t row_word, const uint4& m,
+                                          const unsigned long long* __restrict__ sum, const float* __restrict__ keep, int64_t at) {
+    if (!((row_word | m.x | m.y | m.z | m.w) & kBlkMark)) return false;
+    const float row_sum = (float)__ldg(sum);
     const bool a = blk_faint(v.x, row_word, m.x, row_sum), b = blk_faint(v.y, row_word, m.y, row_sum),
                c = blk_faint(v.z, row_word, m.z, row_sum), d = blk_faint(v.w, row_word, m.w, row_sum);
     if (!(a || b || c || d)) return false;
@@ -227,7 +238,7 @@ struct BlkFinish {
     const uint32_t* col_max;
     const unsigned long long* row_sum;
     const float* keep;
-    unsigned char* again;  // one byte per row of C
+    unsigned char* again;  // one byte per row of C (k_block_tc alone notes them)
 };
 
 // r: columns of a panel.  direct: C, with row stride ldc -- or null, and `fin` is not used.
@@ -313,12 +324,8 @@ k_block_tc(const __half* __restrict__ X, int64_t m_tiles, int64_t k_chunks, cons
                 const int col0 = cur.panel * r + ch * 64;
                 const bool store = !direct || row < rows;
                 uint32_t row_word = 0u;
-                float row_sum = 0.f;
                 bool again = false;
-                if (direct && store) {
-                    row_word = __ldg(fin.row_max + row);
-                    row_sum = (float)__ldg(fin.row_sum + row);
-                }
+                if (direct && store) row_word = __ldg(fin.row_max + row);
                 float* dst = direct ? direct + row * ldc + col0
                                     : partial + (((cur.split * panels + cur.panel) * m_tiles + cur.tile) * 128 + xrow) * (int64_t)r + ch * 64;
 #pragma unroll
@@ -335,7 +342,7 @@ k_block_tc(const __half* __restrict__ X, int64_t m_tiles, int64_t k_chunks, cons
                             if (direct) {
                                 const int col = col0 + g * 16 + j;
                                 const uint4 m = __ldg((const uint4*)(fin.col_max + col));
-                                again = again || blk_again(x, row_word, m, row_sum, fin.keep, row * ldc + col);
+                                again = again || (store && blk_again(x, row_word, m, fin.row_sum + row, fin.keep, row * ldc + col));
                                 x = blk_unscaled4(x, row_word, m);
                             }
                             if (store) *(float4*)(dst + g * 16 + j) = x;
@@ -464,7 +471,7 @@ __global__ void k_fill_blocks(const float* __restrict__ vals, const int32_t* __r
 // either, marked here; sum1, sum2 (zero before): their row_sum (blk_faint), in whole numbers, so that the
 // order of the additions does not matter.  Reads 4 bytes and writes 8 per element.  256 threads; 8
 // consecutive ones write a core matrix.
-// A value that both halves in X2 would lose is left there as their smallest, 2^-35: k_block_repair
+// A value that both halves in X2 would lose is left there as their smallest, 2^-35: blk_repair_row
 // has to see that there is one, and looks it up.
 __global__ void __launch_bounds__(256)
 k_block_split(__half* __restrict__ X1, uint32_t* max1, unsigned long long* sum1, int64_t chunks1, __half* __restrict__ X2,
@@ -605,158 +612,188 @@ struct BlkValues {
     bool columns;
 };
 
-// The rows of C = X * Y whose byte in `again` is set (it is cleared), from the values of X as they are,
-// products and sums in double: what the halves lose of faint values is in these rows
-// too much (blk_faint).  Almost always there are none, and the launch costs a product 3.5 us (3001 x 100003,
-// rank 50).  Where it has to work it is bound by latency: every popular column of 20000 x 4194304 at rank 128 computed
-// again takes 75 ms, the sparse product of the same entries 12.  It stays that way since entries that are
-// this small only last a few updates.  With `columns` the stored entries of a row of X are found
-// through its halves, and the faint ones among them in the row of A.
+// What computing a row of C = X * Y again takes: X's blocks with the words of its rows, its values, Y, and C (M x r).
+struct BlkRepair {
+    const __half* X;
+    const uint32_t* xmax;
+    int64_t k_chunks;
+    BlkValues values;
+    const float* Y;
+    int64_t M, K;
+    int r;
+    float* C;
+};
 constexpr int kRepairThreads = 256, kRepairBatch = 8;
-__global__ void __launch_bounds__(kRepairThreads, 2)
-k_block_repair(const __half* __restrict__ X, const uint32_t* __restrict__ xmax, int64_t k_chunks, const BlkValues ex,
-               const float* __restrict__ Y, int64_t M, int64_t K, int r, float* __restrict__ C, unsigned char* __restrict__ again) {
+struct BlkRepairSums {
+    double of[512];  // (one set that the warps add to in turn: 32 KB for a set each would be the space that the gathers' L1 has)
+};
+
+// Row i of C by a block of kRepairThreads, from the values of X as they are, products and sums in double: what the
+// halves lose of faint values is in this row too much (blk_faint).  There is hardly ever one.  Where there
+// are many it is bound by latency: every popular column of 20000 x 4194304 at rank 128 computed again
+// takes 75 to 85 ms, the sparse product of the same entries 12; entries that are this small last a few updates only.
+// With `columns` the stored entries of a row of X are found through its halves, and the faint ones among them in
+// the row of A.
+__device__ __forceinline__ void blk_repair_row(const BlkRepair& a, int64_t i, BlkRepairSums& sums) {
+    constexpr int kWarps = kRepairThreads / 32;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, quads = a.r >> 2;
+    double acc[4][4];
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+#pragma unroll
+        for (int t = 0; t < 4; t++) acc[q][t] = 0.0;
+    int64_t beg = 0, end = a.K;
+    if (!a.values.dense && !a.values.columns) {
+        beg = a.values.rowptr[i];
+        end = beg + a.values.hot_len[i * a.values.stride];
+    }
+    const float back = blk_unscale(a.xmax[i]);
+    for (int64_t p0 = beg + w * 32; p0 < end; p0 += kRepairThreads) {
+        const int64_t p = p0 + lane;
+        int64_t k = p;
+        float v = 0.f;
+        if (p < end) {
+            if (a.values.dense) {
+                v = a.values.dense[i * a.K + p];
+            } else if (!a.values.columns) {
+                k = a.values.col[p];
+                v = a.values.vals[p];
+            } else {
+                const __half* x = a.X + ((i >> 7) * a.k_chunks + (p >> 6)) * kBlkHalves + blk_canon((int)(i & 127), (int)(p & 63));
+                v = fmaf(__half2float(x[kBlkHalf]), 1.f / kBlkLoScale, __half2float(x[0]));
+            }
+        }
+        if (!a.values.dense && a.values.columns) {
+            uint32_t ask = __ballot_sync(0xffffffffu, v != 0.f && fabsf(v) < kBlkFaint);
+            v *= back;
+            while (ask) {
+                const int src = __ffs(ask) - 1;
+                ask &= ask - 1;
+                const int64_t row = __shfl_sync(0xffffffffu, k, src), first = a.values.rowptr[row];
+                const int64_t last = first + a.values.hot_len[row * a.values.stride];
+                for (int64_t q = first; q < last; q += 32 * kRepairBatch) {
+                    int found = -1;
+#pragma unroll
+                    for (int b = 0; b < kRepairBatch; b++) {
+                        const int64_t at = q + 32 * b + lane;
+                        if (at < last && a.values.col[at] == i) found = b;
+                    }
+                    const uint32_t hit = __ballot_sync(0xffffffffu, found >= 0);
+                    if (!hit) continue;
+                    const int by = __ffs(hit) - 1;
+                    const int b = __shfl_sync(0xffffffffu, found, by);
+                    if (lane == src) v = a.values.vals[q + 32 * b + by];
+                    break;
+                }
+            }
+        }
+        uint32_t live = __ballot_sync(0xffffffffu, v != 0.f);
+        while (live) {
+            double x[kRepairBatch];  // that many entries at a time, so that their rows of Y are on the way together
+            int64_t at[kRepairBatch];
+            int m = 0;
+#pragma unroll
+            for (int b = 0; b < kRepairBatch; b++) {
+                const int src = live ? __ffs(live) - 1 : 0;
+                x[b] = (double)__shfl_sync(0xffffffffu, v, src);
+                at[b] = __shfl_sync(0xffffffffu, k, src) * quads;
+                m += live ? 1 : 0;
+                live &= live - 1;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                if (32 * q >= quads) continue;
+                const int c = lane + 32 * q;
+                float4 f[kRepairBatch];
+#pragma unroll
+                for (int b = 0; b < kRepairBatch; b++) {
+                    f[b] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (b < m && c < quads) f[b] = __ldg((const float4*)a.Y + at[b] + c);
+                }
+#pragma unroll
+                for (int b = 0; b < kRepairBatch; b++) {
+                    if (b >= m) continue;
+                    acc[q][0] = fma(x[b], (double)f[b].x, acc[q][0]);
+                    acc[q][1] = fma(x[b], (double)f[b].y, acc[q][1]);
+                    acc[q][2] = fma(x[b], (double)f[b].z, acc[q][2]);
+                    acc[q][3] = fma(x[b], (double)f[b].w, acc[q][3]);
+                }
+            }
+        }
+    }
+    for (int turn = 0; turn < kWarps; turn++) {
+        if (w == turn) {
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (lane + 32 * q < quads)
+#pragma unroll
+                    for (int t = 0; t < 4; t++) {
+                        double* const s = sums.of + 4 * (lane + 32 * q) + t;
+                        *s = turn == 0 ? acc[q][t] : *s + acc[q][t];
+                    }
+        }
+        __syncthreads();
+    }
+    for (int c = tid; c < a.r; c += kRepairThreads) a.C[i * a.r + c] = (float)sums.of[c];
+    __syncthreads();
+}
+
+// The rows whose byte in `again` is set (it is cleared); the launch costs a product 3.5 us (3001 x 100003, rank 50),
+// so that products of several splits leave it to k_block_reduce.
+__global__ void __launch_bounds__(kRepairThreads, 2) k_block_repair(const BlkRepair a, unsigned char* __restrict__ again) {
     constexpr int kWarps = kRepairThreads / 32;
     __shared__ int64_t list[kRepairThreads];
     __shared__ int listed;
-    __shared__ double sums[kWarps][512];
+    __shared__ BlkRepairSums sums;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     grid_wait();
-    const int quads = r >> 2;
     // 32 consecutive rows per warp and round
-    for (int64_t g0 = (int64_t)blockIdx.x * kWarps; g0 * 32 < M; g0 += (int64_t)gridDim.x * kWarps) {
+    for (int64_t g0 = (int64_t)blockIdx.x * kWarps; g0 * 32 < a.M; g0 += (int64_t)gridDim.x * kWarps) {
         if (tid == 0) listed = 0;
         __syncthreads();
         const int64_t mine = (g0 + w) * 32 + lane;
-        if (mine < M && again[mine]) {
+        if (mine < a.M && again[mine]) {
             again[mine] = 0;
             list[atomicAdd(&listed, 1)] = mine;  // (in any order: the rows do not depend on one another)
         }
         __syncthreads();
         const int n = listed;
-        for (int l = 0; l < n; l++) {
-            const int64_t i = list[l];
-            double acc[4][4];
-#pragma unroll
-            for (int q = 0; q < 4; q++)
-#pragma unroll
-                for (int t = 0; t < 4; t++) acc[q][t] = 0.0;
-            int64_t beg = 0, end = K;
-            if (!ex.dense && !ex.columns) {
-                beg = ex.rowptr[i];
-                end = beg + ex.hot_len[i * ex.stride];
-            }
-            const float back = blk_unscale(xmax[i]);
-            for (int64_t p0 = beg + w * 32; p0 < end; p0 += kRepairThreads) {
-                const int64_t p = p0 + lane;
-                int64_t k = p;
-                float v = 0.f;
-                if (p < end) {
-                    if (ex.dense) {
-                        v = ex.dense[i * K + p];
-                    } else if (!ex.columns) {
-                        k = ex.col[p];
-                        v = ex.vals[p];
-                    } else {
-                        const __half* x = X + ((i >> 7) * k_chunks + (p >> 6)) * kBlkHalves + blk_canon((int)(i & 127), (int)(p & 63));
-                        v = fmaf(__half2float(x[kBlkHalf]), 1.f / kBlkLoScale, __half2float(x[0]));
-                    }
-                }
-                if (!ex.dense && ex.columns) {
-                    uint32_t ask = __ballot_sync(0xffffffffu, v != 0.f && fabsf(v) < kBlkFaint);
-                    v *= back;
-                    while (ask) {
-                        const int src = __ffs(ask) - 1;
-                        ask &= ask - 1;
-                        const int64_t row = __shfl_sync(0xffffffffu, k, src), first = ex.rowptr[row];
-                        const int64_t last = first + ex.hot_len[row * ex.stride];
-                        for (int64_t q = first; q < last; q += 32 * kRepairBatch) {
-                            int found = -1;
-#pragma unroll
-                            for (int b = 0; b < kRepairBatch; b++) {
-                                const int64_t at = q + 32 * b + lane;
-                                if (at < last && ex.col[at] == i) found = b;
-                            }
-                            const uint32_t hit = __ballot_sync(0xffffffffu, found >= 0);
-                            if (!hit) continue;
-                            const int by = __ffs(hit) - 1;
-                            const int b = __shfl_sync(0xffffffffu, found, by);
-                            if (lane == src) v = ex.vals[q + 32 * b + by];
-                            break;
-                        }
-                    }
-                }
-                uint32_t live = __ballot_sync(0xffffffffu, v != 0.f);
-                while (live) {
-                    double x[kRepairBatch];  // that many entries at a time, so that their rows of Y are on the way together
-                    int64_t at[kRepairBatch];
-                    int m = 0;
-#pragma unroll
-                    for (int b = 0; b < kRepairBatch; b++) {
-                        const int src = live ? __ffs(live) - 1 : 0;
-                        x[b] = (double)__shfl_sync(0xffffffffu, v, src);
-                        at[b] = __shfl_sync(0xffffffffu, k, src) * quads;
-                        m += live ? 1 : 0;
-                        live &= live - 1;
-                    }
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        if (32 * q >= quads) continue;
-                        const int c = lane + 32 * q;
-                        float4 f[kRepairBatch];
-#pragma unroll
-                        for (int b = 0; b < kRepairBatch; b++) {
-                            f[b] = make_float4(0.f, 0.f, 0.f, 0.f);
-                            if (b < m && c < quads) f[b] = __ldg((const float4*)Y + at[b] + c);
-                        }
-#pragma unroll
-                        for (int b = 0; b < kRepairBatch; b++) {
-                            if (b >= m) continue;
-                            acc[q][0] = fma(x[b], (double)f[b].x, acc[q][0]);
-                            acc[q][1] = fma(x[b], (double)f[b].y, acc[q][1]);
-                            acc[q][2] = fma(x[b], (double)f[b].z, acc[q][2]);
-                            acc[q][3] = fma(x[b], (double)f[b].w, acc[q][3]);
-                        }
-                    }
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < 4; q++)
-                if (lane + 32 * q < quads)
-#pragma unroll
-                    for (int t = 0; t < 4; t++) sums[w][4 * (lane + 32 * q) + t] = acc[q][t];
-            __syncthreads();
-            for (int c = tid; c < r; c += kRepairThreads) {
-                double t = sums[0][c];
-#pragma unroll
-                for (int k = 1; k < kWarps; k++) t += sums[k][c];
-                C[i * r + c] = (float)t;
-            }
-            __syncthreads();
-        }
+        for (int l = 0; l < n; l++) blk_repair_row(a, list[l], sums);
         __syncthreads();  // (the list is read before it is started anew)
     }
 }
 
-// out[i][:] (rows i < rows, r4 float4 each) = sum over splits s (in index order) of partial[s][panel][i][:],
-// with the operands' scaling taken out.
-__global__ void k_block_reduce(const float* __restrict__ partial, int n_split, int64_t rows_pad, int64_t rows,
-                               int r4, int pn4, const BlkFinish fin, float4* __restrict__ out) {
-    int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// C[i][:] (r / 4 float4 each) = sum over splits s (in index order) of partial[s][panel][i][:],
+// with the operands' scaling taken out.  A block takes whole rows, 256 / (r / 4) of them, and computes those again that want it.
+__global__ void __launch_bounds__(kRepairThreads, 4)
+k_block_reduce(const float* __restrict__ partial, int n_split, int64_t rows_pad, int pn4, const BlkFinish fin, const BlkRepair a) {
+    __shared__ BlkRepairSums sums;
+    __shared__ bool again[32];
+    const int r4 = a.r >> 2, mine = threadIdx.x / r4, c = threadIdx.x - mine * r4, per = kRepairThreads / r4;
+    const int64_t first = (int64_t)blockIdx.x * per, i = first + mine;
+    if (threadIdx.x < 32) again[threadIdx.x] = false;
     grid_wait();
-    if (idx >= rows * r4) return;
-    const int64_t i = idx / r4;
-    const int c = (int)(idx - i * r4), panel = c / pn4;
-    const float4* p = (const float4*)partial + (panel * rows_pad + i) * pn4 + (c - panel * pn4);
-    float4 a = p[0];
-    for (int s = 1; s < n_split; s++) {
-        float4 b = p[(int64_t)s * rows_pad * r4];
-        a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+    bool want = false;
+    float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+    const bool real = mine < per && i < a.M;
+    if (real) {
+        const int panel = c / pn4;
+        const float4* p = (const float4*)partial + (panel * rows_pad + i) * pn4 + (c - panel * pn4);
+        const uint32_t row_word = __ldg(fin.row_max + i);
+        const uint4 m = __ldg((const uint4*)fin.col_max + c);
+        t = p[0];
+        for (int s = 1; s < n_split; s++) {
+            const float4 b = p[(int64_t)s * rows_pad * r4];
+            t.x += b.x; t.y += b.y; t.z += b.z; t.w += b.w;
+        }
+        want = blk_again(t, row_word, m, fin.row_sum + i, fin.keep, 4 * (i * r4 + c));
+        ((float4*)a.C)[i * r4 + c] = blk_unscaled4(t, row_word, m);
     }
-    const uint32_t row_word = __ldg(fin.row_max + i);
-    const uint4 m = __ldg((const uint4*)fin.col_max + c);
-    if (blk_again(a, row_word, m, (float)__ldg(fin.row_sum + i), fin.keep, 4 * idx)) fin.again[i] = 1;
-    out[idx] = blk_unscaled4(a, row_word, m);
+    if (!__syncthreads_or(want)) return;
+    if (want) again[mine] = true;
+    __syncthreads();
+    for (int l = 0; l < per; l++)
+        if (again[l]) blk_repair_row(a, first + l, sums);
 }
 
 // Ranks up to 128 in one panel; 256, 384 and 512 as panels of 128 columns of Y and C.
@@ -824,11 +861,12 @@ inline int block_tc_launch(const BlkOperand& X, const BlockTcPlan& p, const floa
     DN_TRY(launch_overlapped(k_block_tc, dim3((unsigned)std::min<int64_t>(items, (int64_t)kNumSMs)), kBlkThreads, smem, st, X.blocks,
                              p.m_tiles, p.k_chunks, ysplit, pn, p.panels, p.n_split, p.chunks_per_split, stages, partial,
                              tc_tmem_cols(pn), p.n_split > 1 ? (float*)nullptr : C, M, r, fin, wait_limit, err));
+    const BlkRepair repair = {X.blocks, X.max, p.k_chunks, X.values, Y, M, K, r, C};
     if (p.n_split > 1)
-        DN_TRY(launch_overlapped(k_block_reduce, dim3((unsigned)ceil_div(M * (r / 4), 256)), 256, 0, st, partial, p.n_split,
-                                 p.m_tiles * 128, M, r / 4, pn / 4, fin, (float4*)C));
+        return launch_overlapped(k_block_reduce, dim3((unsigned)ceil_div(M, kRepairThreads / (r / 4))), kRepairThreads, 0, st, partial,
+                                 p.n_split, p.m_tiles * 128, pn / 4, fin, repair);
     return launch_overlapped(k_block_repair, dim3((unsigned)std::min<int64_t>(ceil_div(M, kRepairThreads), 2 * kNumSMs)), kRepairThreads, 0,
-                             st, X.blocks, X.max, p.k_chunks, X.values, Y, M, K, r, C, again);
+                             st, repair, again);
 }
 
 }  // namespace dnpeff
