@@ -132,9 +132,8 @@ struct dnpeff_engine {
     void* h_pinned = nullptr;       // kPinnedBytes of page-locked host memory for scalar read-backs
     int64_t hot_nnz = 0;            // stored entries in popular columns
     SpmmPlan plan_csr, plan_csc;
-    // small problems (kernels_small.cuh): output row of every entry of the CSR and of the CSC, carries, partials
-    int32_t* small_row = nullptr;
-    int32_t* small_col = nullptr;
+    // small problems (kernels_small.cuh): cuts of the two sides, carries, partials
+    SmallCut* small_cuts = nullptr;
     float* small_carry = nullptr;
     float* small_partial = nullptr;
     unsigned int* small_barrier = nullptr;
@@ -374,7 +373,7 @@ void free_matrix(dnpeff_engine* e) {
     dev_free(e, e->gram_scratch);
     dev_free(e, e->tc_scratch);
     e->gram_scratch_floats = 0;
-    dev_free(e, e->small_row); dev_free(e, e->small_col); dev_free(e, e->small_carry);
+    dev_free(e, e->small_cuts); dev_free(e, e->small_carry);
     dev_free(e, e->small_partial); dev_free(e, e->small_barrier);
     dev_free(e, e->plan_csr.long_list);
     dev_free(e, e->plan_csc.long_list);
@@ -1275,27 +1274,29 @@ int run_small(dnpeff_engine* e, int iters, int* made) {
     ArenaScope arena_scope(&e->arena);
     const int ld = e->ld;
     DN_TRY(build_csc(e, true));
-    if (!e->WA) DN_TRY(dev_alloc(e, &e->WA, (size_t)(e->ms * ld)));
-    const uint32_t unit = small_unit(e->nnz, ld);
     const size_t partial = (size_t)kNumSMs * ld * ld;
-    if (!e->small_row) {
-        DN_TRY(dev_alloc(e, &e->small_row, (size_t)e->nnz));
-        DN_TRY(dev_alloc(e, &e->small_col, (size_t)e->nnz));
-        DN_TRY(dev_alloc(e, &e->small_carry, (size_t)ceil_div(e->nnz, unit) * ld));
+    // words that a launch counts in: barrier, abort flag, chunks of either Gram matrix, then a flag per worker of either side
+    const size_t most = (size_t)kNumSMs * small_workers_per_block(ld), sync_words = 4 + 2 * most;
+    const int w_workers = small_workers(e->n, e->nnz, ld), h_workers = small_workers(e->ms, e->nnz, ld);
+    if (!e->small_cuts) {
+        DN_TRY(dev_alloc(e, &e->small_cuts, 2 * (most + 1)));
+        DN_TRY(dev_alloc(e, &e->small_carry, 2 * most * ld));
         DN_TRY(dev_alloc(e, &e->small_partial, 2 * partial));
-        DN_TRY(dev_alloc(e, &e->small_barrier, 2));
-        k_small_row_of<<<(unsigned)std::min<int64_t>(ceil_div(e->n, 8), kNumSMs * 8), 256, 0, e->st>>>(e->a_rowptr, e->n,
-                                                                                                 e->small_row);
-        k_small_row_of<<<(unsigned)std::min<int64_t>(ceil_div(e->ms, 8), kNumSMs * 8), 256, 0, e->st>>>(e->c_colptr, e->ms,
-                                                                                                  e->small_col);
+        DN_TRY(dev_alloc(e, &e->small_barrier, sync_words));
+        const uint32_t cost = small_row_cost(ld);
+        k_small_cuts<<<(unsigned)(w_workers / 256 + 1), 256, 0, e->st>>>(e->a_rowptr, (uint32_t)e->n, cost, (uint32_t)w_workers,
+                                                                       e->small_cuts);
+        k_small_cuts<<<(unsigned)(h_workers / 256 + 1), 256, 0, e->st>>>(e->c_colptr, (uint32_t)e->ms, cost, (uint32_t)h_workers,
+                                                                       e->small_cuts + most + 1);
         DN_LAUNCH_CHECK();
         DN_COUNT_LAUNCH(2);
     }
+    unsigned int* const words = e->small_barrier;
     SmallArgs a;
-    a.w = {e->b_vals, e->b_col, e->small_row, e->a_rowptr, (uint32_t)e->nnz, unit, e->n, small_tile_rows(e->n, ld), e->W, e->H,
-           e->AHG, e->small_carry, e->AHG + e->n * ld, e->small_partial, e->small_partial + partial};
-    a.h = {e->c_vals, e->c_row, e->small_col, e->c_colptr, (uint32_t)e->nnz, unit, e->ms, small_tile_rows(e->ms, ld), e->H, e->W,
-           e->WA, e->small_carry, e->WW, e->small_partial + partial, e->small_partial};
+    a.side[0] = {e->b_vals, e->b_col, e->a_rowptr, e->small_cuts, (uint32_t)w_workers, e->W, e->H, e->small_carry, words + 4,
+           e->AHG + e->n * ld, words + 2, e->small_partial, 0, e->small_partial + partial};
+    a.side[1] = {e->c_vals, e->c_row, e->c_colptr, e->small_cuts + most + 1, (uint32_t)h_workers, e->H, e->W, e->small_carry + most * ld,
+           words + 4 + most, e->WW, words + 3, e->small_partial + partial, 0, e->small_partial};
     a.r4 = (e->p.rank + 3) / 4;
     a.eps = e->p.eps;
     a.barrier = e->small_barrier;
@@ -1304,7 +1305,7 @@ int run_small(dnpeff_engine* e, int iters, int* made) {
     for (*made = 0; *made < iters; *made += a.iters) {
         a.iters = std::min(kSmallIters, iters - *made);
         bool launched = false;
-        DN_TRY(small_launch(a, ld, e->st, e->opt_refuse_cooperative, &launched));
+        DN_TRY(small_launch(a, ld, sync_words, e->st, e->opt_refuse_cooperative, &launched));
         if (!launched) break;
     }
     return DNPEFF_OK;

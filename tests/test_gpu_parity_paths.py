@@ -333,6 +333,42 @@ def test_small_problems_in_one_launch(torch_cuda, n, m, lens, r):
     assert rel_fro(got[0][0], Ws) < 1e-5 and rel_fro(got[0][1], Hs) < 1e-5
 
 
+@pytest.mark.parametrize("n,m,lens,r", [
+    (65, 3000, (40, 41), 96), (129, 2600, (1, 60), 128),      # a row more than a tile, or a half, of the wide strides
+    (600, 900, (300, 301), 100), (2400, 70, (30, 60), 96),    # rows cut over many workers; more rows than tiles on W's side
+    (40, 50000, (2000, 2100), 64), (16, 20000, (6000, 6001), 128)])  # several tiles a worker on H's
+def test_small_problem_tiles_and_tiny_values(torch_cuda, n, m, lens, r):
+    """The one-launch kernel around its tiles and cuts, and with components so small that numerators fall below 2^-100
+    and below the normal range: against single steps and the oracle."""
+    from npeff_ref_b200 import MuNmfParams
+    rng = np.random.default_rng(n + m + r)
+    vals, ind, ptr = _ragged(rng, n, m, rng.integers(lens[0], lens[1], size=n))
+    iters, eps = 3, 1e-8
+    with _engine(MuNmfParams(rank=r, eps=eps, seed=6, init_scale=0.3)) as eng:
+        eng.set_csr(n, m, vals, ind, ptr, 0, None, 1)
+        mk = eng.shape[1]
+        W0, H0 = O.init_factors(n, mk, r, 6, 0.3)
+        H0[::5] *= np.float32(1e-33)
+        H0[1::7] *= np.float32(1e-38)
+        eng.init_factors(W0, H0)
+        eng.run(iters, log_every=0)
+        got = eng.load_w_to_host(), eng.load_h_to_host()
+        eng.init_factors(W0, H0)
+        for _ in range(iters):
+            eng.step_w()
+            eng.step_h()
+        Ws, Hs = eng.load_w_to_host(), eng.load_h_to_host()
+    v, c, rp, n2o = O.prune_columns(vals, ind, ptr, m, 1)
+    Wo, Ho, _ = O.run(v, c, rp, mk, W0, H0, iters, eps, acc64=True, losses=True)
+    for g, s, o in ((got[0], Ws, Wo), (got[1], Hs, Ho)):
+        assert rel_fro(g, o) < 1e-5 and rel_fro(g, s) < 1e-5
+        assert np.isfinite(g).all()
+    # Entry by entry: an update is good to a few 1e-6 (numerator and denominator are sums of positive terms: 2^-24 times the
+    # square root of their number and more, and the tensor core's 6e-7), three updates of either factor to 4e-5; the last place of
+    # the subnormal range, 2^-149, once an update and factor
+    assert np.allclose(got[1], Ho, rtol=4e-5, atol=1e-44), np.abs(got[1] - Ho).max()
+
+
 def test_small_problem_barrier_wait_runs_out(torch_cuda):
     """With a wait limit of one poll the grid barrier of the small-problem kernel gives up, every
     block leaves, the status says so, and the engine works again with the default limit."""
