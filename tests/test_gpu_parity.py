@@ -153,6 +153,24 @@ def test_op_mu_update_zero_and_tiny_numerators(torch_cuda, rows, r):
     assert np.allclose(got, want, rtol=3e-6, atol=1e-44), np.abs(got - want).max()
 
 
+@pytest.mark.parametrize("rows,r", [(1, 256), (129, 384), (4737, 512), (6273, 384), (9473, 256), (18945, 256)])
+def test_op_mu_update_wide_panel_split(torch_cuda, rows, r):
+    """Wide updates around the row counts where a tile's panels go to one block, to two, or to one each, against float64.
+    Bound: the operator's denominators hold 3e-6, the division and the product a unit in the last place each."""
+    from npeff_ref_b200._lib import lib, check
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(rows + r)
+    X, Num = (torch.rand((rows, r), generator=g, device="cuda") for _ in range(2))
+    B = torch.rand((r + 3, r), generator=g, device="cuda")
+    G = B.T @ B
+    G = (G + G.T) / 2
+    want = X.double() * (Num.double() / (X.double() @ G.double() + 1e-8))
+    check(lib().dnpeff_op_mu_update(X.data_ptr(), Num.data_ptr(), G.data_ptr(), rows, r, 1e-8,
+                                    torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    assert ((X.double() - want).abs() <= 4e-6 * want.abs()).all()
+
+
 # ---------------------------------------------------------------------------
 @pytest.mark.parametrize("min_count", [1, 2, 3])
 @pytest.mark.parametrize("n_shards", [1, 3])
