@@ -176,9 +176,10 @@ __device__ __forceinline__ void gsplit_store(float* __restrict__ Gsplit, int r, 
 // itself, took 13 to 20 us of latency (64 KB of partials at rank 32, 9.7 MB at 128); 3 to 5 this
 // way.  The lower triangle is a copy, so that the result is symmetric bit for bit.  Gsplit (or
 // NULL): the same matrix split for the update kernel, which saves that a launch.
+// A partial (of one tile) may hold 1 << fold Gram matrices on its diagonal, all of them to be added.
 static __global__ void __launch_bounds__(256)
 k_gram_reduce(const float* __restrict__ partial, int nslab, int npairs, int ntile, int tile, int r,
-              float* __restrict__ G, float* __restrict__ Gsplit) {
+              float* __restrict__ G, float* __restrict__ Gsplit, int fold) {
     __shared__ double sums[8][32];
     grid_wait();
     const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
@@ -192,7 +193,7 @@ k_gram_reduce(const float* __restrict__ partial, int nslab, int npairs, int ntil
         const float* p = partial + (int64_t)pair * (tile * tile) + (a % tile) * tile + b % tile;
         const int64_t stride = (int64_t)npairs * (tile * tile);
 #pragma unroll 4
-        for (int sl = y; sl < nslab; sl += 8) s += (double)p[sl * stride];
+        for (int sl = y; sl < nslab << fold; sl += 8) s += (double)p[(sl >> fold) * stride + (sl & ((1 << fold) - 1)) * (r * tile + r)];
     }
     sums[y][x] = s;
     __syncthreads();
@@ -209,9 +210,9 @@ k_gram_reduce(const float* __restrict__ partial, int nslab, int npairs, int ntil
 }
 
 inline int gram_reduce_launch(const float* partial, int nslab, int npairs, int ntile, int tile, int r, float* G,
-                              float* Gsplit, cudaStream_t st) {
+                              float* Gsplit, cudaStream_t st, int fold = 0) {
     return launch_overlapped(k_gram_reduce, dim3((unsigned)ceil_div((int64_t)r * r, 32)), 256, 0, st, partial, nslab, npairs, ntile,
-                             tile, r, G, Gsplit);
+                             tile, r, G, Gsplit, fold);
 }
 
 struct GramPlan {

@@ -104,6 +104,21 @@ def test_op_gram_matches_oracle(torch_cuda, rows, r):
     assert np.array_equal(got, got.T)
 
 
+@pytest.mark.parametrize("rows,r", [(303103, 32), (303104, 32), (303107, 32), (400001, 32), (151551, 64), (151552, 64), (151617, 64)])
+def test_op_gram_folded_rows(torch_cuda, rows, r):
+    """Around the row count from which several rows of a narrow X are one of 128 columns: whole and cut last rows, against
+    float64 to the bound of the test above."""
+    from npeff_ref_b200._lib import lib, check
+    torch = torch_cuda
+    X = torch.rand((rows, r), generator=torch.Generator(device="cuda").manual_seed(rows), device="cuda")
+    G = torch.full((r, r), float("nan"), device="cuda")
+    check(lib().dnpeff_op_gram(X.data_ptr(), rows, r, G.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    want = X.double().T @ X.double()
+    assert ((G.double() - want).abs() <= 3e-6 * want.max()).all()
+    assert torch.equal(G, G.T)
+
+
 @pytest.mark.parametrize("rows,r", [(1, 4), (513, 32), (300, 64), (1000, 48), (4099, 128),
                                     (700, 256), (200, 512), (3000, 384), (50, 5), (64, 516),
                                     (40001, 128), (60000, 64),    # several tiles per block
