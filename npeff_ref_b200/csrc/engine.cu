@@ -1040,7 +1040,7 @@ int fill_csc(dnpeff_engine* e, int mode) {
     {
         int64_t blocks = std::min<int64_t>(ceil_div(col_last - col_first, 8), (int64_t)kNumSMs * 32);
         k_csc_order_short<<<(unsigned)blocks, 256, 0, st>>>(e->c_colptr, col_first, col_last, tvals, trow,
-                                                           cvals, crows, err.p);
+                                                           cvals, crows, e->n, err.p);
         DN_LAUNCH_CHECK();
         DN_COUNT_LAUNCH(2);
     }

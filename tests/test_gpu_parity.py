@@ -104,6 +104,32 @@ def test_op_gram_matches_oracle(torch_cuda, rows, r):
     assert np.array_equal(got, got.T)
 
 
+@pytest.mark.parametrize("n", [600, 8192, 8193])
+def test_csc_row_order_by_column_length(torch_cuda, n):
+    """Columns of lengths around what the row order is found by (pairs, in fours; a bitmap of at most 8192 rows; a block from 513
+    entries on): bit for bit the stable transpose, and a repeated column of a row is found in each."""
+    from npeff_ref_b200 import MuNmfParams, DnpeffError
+    rng = np.random.default_rng(n)
+    lens = [1, 2, 3, 4, 5, 11, 16, 17, 31, 32, 33, 63, 64, 65, 129, 255, 256, 257, 509, 511, 512, 513, 600]
+    pairs = np.concatenate([np.stack([rng.choice(n, length, replace=False), np.full(length, c)], 1) for c, length in enumerate(lens)])
+    pairs = pairs[rng.permutation(len(pairs))]          # a row's columns in any order
+    pairs = pairs[np.argsort(pairs[:, 0], kind="stable")]
+    ptr = np.concatenate([[0], np.cumsum(np.bincount(pairs[:, 0], minlength=n))]).astype(np.int64)
+    ind, vals = pairs[:, 1].astype(np.int32), rng.random(len(pairs), dtype=np.float32) + np.float32(0.1)
+    with _engine(MuNmfParams(rank=8), keep_csr=True) as eng:
+        eng.set_csr(n, len(lens), vals, ind, ptr, 0, None, 1)
+        v, c, rp = eng.export_shard_csr()
+        for got, want in zip(eng.export_shard_csc(), O.csr_to_csc(v, c, rp, len(lens))):
+            assert np.array_equal(got, want)
+        for length in (5, 64, 511):                     # the row of a column's first entry gets that column twice
+            at = int(np.flatnonzero(ind == lens.index(length))[0])
+            row = int(np.searchsorted(ptr, at, side="right")) - 1
+            ptr2 = ptr + (np.arange(n + 1) > row)
+            eng.set_csr(n, len(lens), np.insert(vals, at, vals[at]), np.insert(ind, at, ind[at]), ptr2, 0, None, 1)
+            with pytest.raises(DnpeffError, match="twice"):
+                eng.export_shard_csc()
+
+
 @pytest.mark.parametrize("rows,r", [(303103, 32), (303104, 32), (303107, 32), (400001, 32), (151551, 64), (151552, 64), (151617, 64)])
 def test_op_gram_folded_rows(torch_cuda, rows, r):
     """Around the row count from which several rows of a narrow X are one of 128 columns: whole and cut last rows, against
