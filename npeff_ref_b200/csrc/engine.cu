@@ -1266,7 +1266,7 @@ int step_h(dnpeff_engine* e) {
 bool small_problem(const dnpeff_engine* e) {
     if (!tensor_cores_enabled() || e->timing || e->p.n_shards > 1 || !small_rank_ok(e->ld)) return false;
     if (e->n <= 0 || e->ms <= 0 || e->nnz <= 0 || e->nnz > ((int64_t)1 << 30)) return false;
-    return small_pays(e->nnz, e->n + e->ms, (e->p.rank + 3) / 4, e->ld);
+    return small_pays(e->nnz, e->n + e->ms, e->ld, e->hot_nnz, e->n * e->n_hot);
 }
 
 // *made: iterations that were made; fewer than asked for where the launch was refused.

@@ -963,17 +963,27 @@ inline int small_workers(int64_t rows, int64_t entries, int ld) {
 // Whether these launches beat the large path.  An iteration takes about 15 us, two gathers of a factor row per stored entry, and the two
 // contractions.  The large path takes 65 to 105 us plus the same gathers, but does the popular columns densely and contracts at the
 // tensor cores' full rate.  us an iteration here and there:
-//   stride 32: 8000 x 600000 x 4000 values 652, 792; 500 x 600000 x 20000 341, 501; 12000 x 100000 x 3000 560, 557
+//   stride 32: 8000 x 600000 x 4000 values 694, 795; 500 x 600000 x 20000 341, 501; 17000 x 200000 x 1800 525, 570; 3000 x 60000 x 4000
+//              213, 237; 20000 x 50000 x 1500 477, 454; 5000 x 20000 x 3000 239, 221
 //   64: 2000 x 40000 x 2000 168, 171; 1000 x 200000 x 2000 221, 227; 5000 x 50000 x 1000 203, 191; 3001 x 100003 x 2047 312, 250
 //   96: 12000 x 12000 x 150 142, 165; 200 x 100000 x 3000 144, 169; 3060 x 80340 x 368 176, 170; 1500 x 60000 x 1500 217, 205
 //   128: 800 x 40000 x 1000 118, 172; 200 x 100000 x 3000 159, 181; 4000 x 40000 x 300 160, 160; 828 x 74164 x 8240 560, 284
-inline bool small_pays(int64_t nnz, int64_t rows, int r4, int ld) {
-    // bytes gathered per us, elements contracted per us, and where the large path takes over
-    const double gather = ld <= 64 ? 15.0e6 : (ld == 96 ? 11.0e6 : 12.0e6);
-    const double contract = ld == 32 ? 5.0e6 : (ld == 64 ? 6.5e6 : (ld == 96 ? 10.0e6 : 20.0e6));
-    const double line = ld == 32 ? 620.0 : (ld == 64 ? 205.0 : (ld == 96 ? 166.0 : 155.0));
-    const double bytes = ld == 32 ? 16.0 * r4 : 4.0 * ld;  // (a lane group takes whole strides)
-    return 15.0 + 2.0 * (double)nnz * bytes / gather + (double)rows * ld * ld / contract < line;
+// popular: stored entries in popular columns; block: elements of the dense block.
+inline bool small_pays(int64_t nnz, int64_t rows, int ld, int64_t popular, int64_t block) {
+    if (ld == 32) {
+        // Here large problems can gain too, and what decides is how dense the popular columns are.  us per million gathers, per MB of
+        // the dense block and per MB of factors and numerators, from fourteen shapes (here within 3 %, there 8, but for the least): the
+        // large path where the two are about even.
+        const double gathers = 2e-6 * (double)nnz, factors = 384e-6 * (double)rows;
+        const double here = 7.5 * gathers + 0.84 * factors;
+        const double there = 73.0 + 6.8 * 2e-6 * (double)(nnz - popular) + 0.18 * 8e-6 * (double)block + 1.47 * factors;
+        return 1.04 * here < there;
+    }
+    // bytes gathered per us (a lane group takes whole strides), elements contracted per us, and where the large path takes over
+    const double gather = ld == 64 ? 15.0e6 : (ld == 96 ? 11.0e6 : 12.0e6);
+    const double contract = ld == 64 ? 6.5e6 : (ld == 96 ? 10.0e6 : 20.0e6);
+    const double line = ld == 64 ? 205.0 : (ld == 96 ? 166.0 : 155.0);
+    return 15.0 + 8.0 * ld * (double)nnz / gather + (double)rows * ld * ld / contract < line;
 }
 
 // All blocks have to be on the GPU together: where the process may not use that many SMs (a share of an MPS
