@@ -64,7 +64,7 @@ struct SmallShape {
     static constexpr int kLdN = LD + 4;                        // row strides in shared memory: numerators,
     static constexpr int kLdX = LD + 4;                        // and X
     static constexpr int kSub = kWide ? 1 : kT / (kQuads * kQuads);  // threads of a square of the Gram matrix on CUDA cores
-    static constexpr int kVec = LD > 64 ? 4 : 1;                 // elements per lane of a chunk of G
+    static constexpr int kVec = kWide ? 4 : 1;                 // elements per lane of a chunk of G
     static constexpr int kChunks = LD * LD / (32 * kVec);
     // a worker's shared memory, in floats: G, and X (wide: the operand in shared memory, X or X^T in halves) | numerators |
     // carries, the last one of the piece of another worker's row | sums of the Gram matrix (narrow) | row offsets, of either
@@ -977,7 +977,7 @@ inline bool small_pays(int64_t nnz, int64_t rows, int ld, int64_t popular, int64
         const double gathers = 2e-6 * (double)nnz, factors = 384e-6 * (double)rows;
         const double here = 7.5 * gathers + 0.84 * factors;
         const double there = 73.0 + 6.8 * 2e-6 * (double)(nnz - popular) + 0.18 * 8e-6 * (double)block + 1.47 * factors;
-        return 1.04 * here < there;
+        return nnz <= (1 << 26) && rows <= (1 << 22) && 1.04 * here < there;  // (not looked at beyond)
     }
     // bytes gathered per us (a lane group takes whole strides), elements contracted per us, and where the large path takes over
     const double gather = ld == 64 ? 15.0e6 : (ld == 96 ? 11.0e6 : 12.0e6);
