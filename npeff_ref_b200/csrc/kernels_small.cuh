@@ -316,9 +316,10 @@ __device__ __forceinline__ void small_add_pieces(F& x, const SmallArgs& a, const
     }
 }
 
-// Few partials: the worker sums all of G for itself.  In a fixed order and in double, as below.
+// Few partials (8 at stride 32, 2 at 64): the worker sums all of G for itself.  In a fixed order and in double, as below.  (us an iteration
+// at 8 and 32: 185 x 2695, rank 12, 14.1, 17.2; 64 x 2048, rank 32, 16.4, 18.2; 64 of them 24 and 18.)
 template <int LD>
-__device__ __forceinline__ bool small_gram_direct(int partials) { return !SmallShape<LD>::kWide && partials * LD * LD <= 32768  /* 128 KB */; }
+__device__ __forceinline__ bool small_gram_direct(int partials) { return !SmallShape<LD>::kWide && partials * LD * LD <= 8192; }
 template <int LD>
 __device__ __forceinline__ void small_gram_sum_all(const SmallSide& s, int t, float* G) {
     for (int e = t; e < LD * LD / 2; e += SmallShape<LD>::kT) {
@@ -951,13 +952,13 @@ inline int small_workers_per_block(int ld) { return ld > 64 ? 1 : 2; }
 // 172, 167, 167; 1738 x 186396 x 3055 values, 32, 159, 154, 161; 300 x 9000 x 1500, 128, 60, 60, 61; 832 x 11990 x 1199, 94, 97, 89, 89).
 inline uint32_t small_row_cost(int ld) { return (uint32_t)(ld <= 64 ? 8 + ld / 2 : 4 + ld / 3); }
 
-// Workers of a side: as many as there are, but each with the work of 1024 gathers, or 384 at the wide strides, whose tiles take time by
-// runs of 16 rows (64 x 2048, rank 32: 18 us an iteration at 512 or 768, 16 at 1024, 21 at 2048, 27 at 4096; 585 x 3702, rank 48: 24,
-// 25, 25, 28, 43; 458 x 2551, rank 96: 32 at 384, 36 at 1024).
+// Workers of a side: as many as there are, but each with the work of 600 gathers, or 384 at the wide strides, whose tiles take time by
+// runs of 16 rows (us an iteration at 600 and 1024: 185 x 2695, rank 12, 14.1, 15.5; 969 x 6722, rank 33, 27.2, 29.6; 64 x 2048, rank 32,
+// 16.4, 15.8, and 20 or more from 1500 on; 458 x 2551, rank 96: 32 at 384, 36 at 1024).
 inline int small_workers(int64_t rows, int64_t entries, int ld) {
     const int64_t cost = entries + rows * small_row_cost(ld);
     const int64_t most = (int64_t)kNumSMs * small_workers_per_block(ld);
-    return (int)std::min(most, std::max<int64_t>(1, cost / (ld > 64 ? 384 : 1024)));
+    return (int)std::min(most, std::max<int64_t>(1, cost / (ld > 64 ? 384 : 600)));
 }
 
 // Whether these launches beat the large path.  An iteration takes about 15 us, two gathers of a factor row per stored entry, and the two
