@@ -25,7 +25,7 @@
 //
 // Sparse products.  The entries of a tile are cut into equal units, one per lane group (LD / 4 lanes, a
 // float4 of the factor row each: with two float4 a lane and rows of 128 bytes every load would touch eight lines for
-// four, 1.2 times the time); a unit adds up its entries row by row.  The sum of a row that starts
+// four, 1.2 times the time); a unit adds up its entries row by row, in runs of at most kSmallRun.  The sum of a row that starts
 // inside the unit goes to the row's place, the sum of one that started earlier to the unit's carry slot,
 // and whoever reads a row adds the carries of the units that begin inside it, in order.  So a row of two
 // thousand entries and two thousand rows of one entry take the same time, and the result does not depend
@@ -179,7 +179,18 @@ struct SmallSum {             // of a unit's row: this lane's float4
         small_fma2(x[0], v, make_float2(a.x, a.y));
         small_fma2(x[1], v, make_float2(a.z, a.w));
     }
+    __device__ __forceinline__ void add(const SmallSum& s) {
+        small_fma2(x[0], 1.f, s.x[0]);
+        small_fma2(x[1], 1.f, s.x[1]);
+    }
 };
+
+// A unit adds up runs of at most this many entries, and then the runs: where a worker's tile has 10^5 entries its units have thousands,
+// and one chain of them is off by 2^-24 times the square root of their number.  Numerators of W against float64 (rms after two updates; one
+// chain, runs of 64): 8000 x 600000 x 4000 values, rank 32, 7.2e-7, 1.2e-7; 17000 x 200000 x 1800 8.6e-7, 1.4e-7; on the large path
+// 5.1e-7 and 5.2e-7.  us an iteration: 693, 704 and 571, 578; 500 x 600000 x 20000 349, 356; 2048 x 65536 x 4096 160.7, 161.8;
+// 300 x 9000 x 1500, rank 128, 59.4, 59.4.  (The loop counts down: a register less, 1 % at 32 and 64 and 2 at 96 and 128.)
+constexpr uint32_t kSmallRun = 64;
 
 // Where the units of a tile whose entries begin at e0 begin.
 template <int LD>
@@ -227,10 +238,16 @@ __device__ __forceinline__ void small_gather(const SmallSide& s, const SmallTile
     float* dst = ((i >= 0 ? sp[i] : tl.e0) < beg ? C + g * LD : (i >= 0 ? N + i * S::kLdN : C + S::kUnits * LD)) + 4 * q;
     bool started = false;
     uint32_t i_end = tl.rows > 0 ? sp[i + 1] : tl.e1;
-    SmallSum acc;
+    SmallSum acc, runs;  // of the row: the present run of entries, and the runs before
     acc.clear();
+    runs.clear();
     constexpr uint32_t kFirst = kLanes == 8 ? 0x01010101u : (kLanes == 16 ? 0x00010001u : 1u);  // the first lanes of a warp's units
-    for (uint32_t off = 0; off < unit; off += kB, p += kB) {  // the same trips for every unit of the warp
+    static_assert(kSmallRun % kB == 0, "a run ends with a batch");
+    for (uint32_t left = unit; left != 0; left -= kB, p += kB) {  // the same trips for every unit of the warp
+        if (left % kSmallRun == 0) {
+            runs.add(acc);
+            acc.clear();
+        }
         const bool in = q < kB && p + q >= beg && p + q < end;
         float4 h[kB];
         fetch(p + kB, vn, jn);
@@ -264,6 +281,8 @@ __device__ __forceinline__ void small_gather(const SmallSide& s, const SmallTile
                     const int row = __shfl_sync(0xffffffffu, i, k, kLanes);
                     if (lasts >> ((threadIdx.x & 31u) - q + k) & 1u) {
                         if (started) dst = N + row * S::kLdN + 4 * q;
+                        acc.add(runs);
+                        runs.clear();
                         if (q < kQuads) *(float4*)dst = real ? make_float4(acc.x[0].x, acc.x[0].y, acc.x[1].x, acc.x[1].y) : make_float4(0.f, 0.f, 0.f, 0.f);
                         started = true;
                         acc.clear();

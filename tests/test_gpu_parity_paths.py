@@ -369,6 +369,51 @@ def test_small_problem_tiles_and_tiny_values(torch_cuda, n, m, lens, r):
     assert np.allclose(got[1], Ho, rtol=4e-5, atol=1e-44), np.abs(got[1] - Ho).max()
 
 
+@pytest.mark.parametrize("n,m,k,r", [(8000, 1200000, 4000, 32), (17000, 200000, 1800, 20)])
+def test_small_problem_long_sums_against_float64(torch_cuda, n, m, k, r):
+    """The one-launch kernel with some 3e7 entries: tens of tiles a worker on H's side, rows of thousands of entries on W's, and
+    units of one and a half to two thousand entries a row or less.  Two iterations against float64: a numerator is a
+    sum of chains of 64 and then of at most some 60 positive terms, off by 2^-24 * 0.5 * sqrt(124 / 3) = 2e-7 at one standard
+    deviation of the roundings (half of it measured), and two numerators of either factor go into the result; one
+    chain of two thousand alone would be off by 7e-7."""
+    from npeff_ref_b200 import MuNmfParams
+    from npeff_ref_b200._lib import lib, check
+    torch = torch_cuda
+    vals = torch.empty((n, k), dtype=torch.float32, device="cuda")
+    idx = torch.empty((n, k), dtype=torch.int32, device="cuda")
+    norms = torch.empty((n,), dtype=torch.float32, device="cuda")
+    check(lib().dnpeff_synth_pef_device(n, m, k, 1.1, 1.0, 5, vals.data_ptr(), idx.data_ptr(), norms.data_ptr(),
+                                        torch.cuda.current_stream().cuda_stream))
+    vals /= norms[:, None]
+    torch.cuda.synchronize()
+    eps = 1e-12
+    with _engine(MuNmfParams(rank=r, eps=eps, seed=3)) as eng:
+        eng.set_csr_device(n, m, vals.data_ptr(), idx.data_ptr(), 0, k, 0, 1)
+        mk = eng.shape[1]
+        eng.set_init_scale((eng.a_sum() / (n * mk) / r) ** 0.5)
+        for _ in range(2):
+            eng.init_factors()
+            W0, H0 = eng.load_w_to_host(), eng.load_h_to_host()
+            launches = eng.launch_count()
+            eng.run(2, log_every=0)
+            launches = eng.launch_count() - launches
+        assert launches == 1
+        got = [torch.from_numpy(x).cuda() for x in (eng.load_w_to_host(), eng.load_h_to_host().T.copy())]
+        to_kept = torch.zeros(m, dtype=torch.int64, device="cuda")
+        to_kept[torch.from_numpy(eng.new_to_og()).cuda().long()] = torch.arange(mk, device="cuda")
+    W, H = (torch.from_numpy(x).cuda().double() for x in (W0, H0.T.copy()))
+    parts = [(to_kept[idx[a:a + 1000].long()], vals[a:a + 1000].double()) for a in range(0, n, 1000)]
+    for _ in range(2):
+        num = torch.cat([torch.bmm(v.unsqueeze(1), H[c.reshape(-1)].reshape(*c.shape, r))[:, 0] for c, v in parts])
+        W = W * (num / (W @ (H.T @ H) + eps))
+        num = torch.zeros_like(H)
+        for (c, v), w in zip(parts, W.split(1000)):
+            num.index_add_(0, c.reshape(-1), (v.unsqueeze(2) * w.unsqueeze(1)).reshape(-1, r))
+        H = H * (num / (H @ (W.T @ W) + eps))
+    for g, want in zip(got, (W, H)):
+        assert float((g.double() - want).norm() / want.norm()) < 3e-7
+
+
 def test_small_problem_barrier_wait_runs_out(torch_cuda):
     """With a wait limit of one poll the grid barrier of the small-problem kernel gives up, every
     block leaves, the status says so, and the engine works again with the default limit."""
