@@ -123,9 +123,9 @@ k_gram_partial(const float* __restrict__ X, int64_t rows, int r, int ntile, int6
 // with two warps per scheduler: 1.11 ms for the mean update of configuration 2 against 1.03);
 // these interleave.  It needs t below 2^100 or so (else r is flushed), |n| >= 2^-100 (else the
 // residual loses bits) and a finite quotient: callers check a batch afterwards -- a quotient
-// that is infinite or NaN, or r or a dividend other than zero below 2^-100 -- and send the
-// warp through the IEEE division for that batch.  Outside these checks only quotients below
-// 2^-126 can be less accurate.
+// that is infinite or NaN, or r or a dividend other than zero below 2^-100 -- and do the whole
+// batch again with quot_careful.  Outside these checks only quotients below 2^-126 can be less
+// accurate: within 1.5 * 2^-149.
 __device__ __forceinline__ float quot_refined(float n, float t, float& r) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(t));
     const float q = __fmul_rn(n, r);
@@ -140,8 +140,9 @@ __device__ __forceinline__ bool quot_doubtful(float chk, float r_min, uint32_t l
 
 // n / t in a doubtful batch.  Most are in doubt for a dividend below 2^-100 (factor entries on their
 // way to zero, and with heavy-tailed values many at once): those go by 2^60 times the dividend, which is exact and so is the way
-// back unless the quotient is subnormal; the rest takes the IEEE division, whose slow path is a call (458 x 2551, rank 96,
-// heavy-tailed values: an update of 25 rows took 8 us for 3.5).
+// back unless the quotient is subnormal.  Members that were not in doubt come out bit for bit as they were.  What is left -- divisors
+// above 2^99, quotients that are not finite or would be subnormal on the way back -- takes the IEEE division, whose slow path is a call
+// (458 x 2551, rank 96, heavy-tailed values: an update of 25 rows took 8 us for 3.5).  The bound of quot_refined holds for all operands.
 __device__ __forceinline__ float quot_careful(float n, float t) {
     constexpr float k2p60 = 1152921504606846976.f;
     const bool tiny = 2u * __float_as_uint(n) - 1u < 2u * (27u << 23) - 1u, common = t <= 6.338253e29f;  // 2^99
