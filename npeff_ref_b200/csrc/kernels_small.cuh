@@ -74,6 +74,12 @@ struct SmallShape {
                          kC = kN + kTile * kLdN, kS = kC + (kUnits + 1) * LD, kP = kS + (kWide ? 0 : LD * LD),
                          kR = kP + 4 * kOffsets, kFloats = kR + kTile;
     static_assert(2 * kWarps * 32 * kVec <= kS - kN, "the chunk sums (doubles) go over numerators and carries");
+    // Dynamic shared memory of a block.  A block of the wide strides holds all of its SM's TMEM and waits for blocks on other SMs: of two
+    // launches (of two engines) that shared SMs, each could hold TMEM that the other waits for.  So it takes more than half of an SM's
+    // 228 KB, whatever its registers are.
+    static constexpr size_t kNeeds = sizeof(float) * kFloats * kWorkers, kSmem = kWide && kNeeds < 120 * 1024 ? 120 * 1024 : kNeeds;
+    static_assert(!kWide || 2 * kSmem > 228 * 1024, "one block per SM");
+    static_assert(kSmem <= 226 * 1024, "and the static arrays beside it");
 };
 
 // Wide strides, TMEM columns: G as hi | lo, then the runs of either product, then X^T as hi | lo.
@@ -1012,11 +1018,10 @@ inline bool small_pays(int64_t nnz, int64_t rows, int ld, int64_t popular, int64
 template <int LD>
 inline int small_launch_t(SmallArgs& a, int blocks, cudaStream_t st, bool refuse, bool* made) {
     using S = SmallShape<LD>;
-    constexpr size_t smem = sizeof(float) * S::kFloats * S::kWorkers;
-    DN_CUDA(cudaFuncSetAttribute(k_small_run<LD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    DN_CUDA(cudaFuncSetAttribute(k_small_run<LD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::kSmem));
     void* args[] = {&a};
     const cudaError_t e = refuse ? cudaErrorCooperativeLaunchTooLarge
-                                 : cudaLaunchCooperativeKernel((void*)k_small_run<LD>, dim3((unsigned)blocks), dim3(S::kThreads), args, smem, st);
+                                 : cudaLaunchCooperativeKernel((void*)k_small_run<LD>, dim3((unsigned)blocks), dim3(S::kThreads), args, S::kSmem, st);
     *made = e != cudaErrorCooperativeLaunchTooLarge;
     if (!*made) {
         cudaGetLastError();

@@ -437,6 +437,41 @@ def test_small_problem_barrier_wait_runs_out(torch_cuda):
         assert np.array_equal(eng.load_w_to_host(), want)
 
 
+def test_small_problems_of_two_engines_at_once(torch_cuda):
+    """Two threads with an engine and a stream each, at the strides whose blocks hold all of an SM's TMEM: launches of the
+    one-launch kernel queue up behind one another (a block takes more than half of an SM's shared memory) and give
+    the same bits as one engine after the other."""
+    import threading
+    from npeff_ref_b200 import MuNmfParams
+    torch = torch_cuda
+    problems = [(300, 9000, 1500, 128), (200, 20000, 600, 96)]
+    inputs = [make_problem(n, m, k, seed=n + r) for n, m, k, r in problems]
+    got = [[], []]
+
+    def job(i, runs, out):
+        n, m, k, r = problems[i]
+        vals, idx, norms = inputs[i]
+        stream = torch.cuda.Stream()
+        with _engine(MuNmfParams(rank=r, eps=1e-8, seed=6, init_scale=0.05), stream=stream.cuda_stream) as eng:
+            eng.set_csr(n, m, vals, idx, None, k, norms, 1)
+            for _ in range(runs):
+                eng.init_factors()
+                eng.run(100, log_every=0)
+                out.append((eng.load_w_to_host(), eng.load_h_to_host()))
+
+    for i in range(2):
+        job(i, 1, got[i])
+    threads = [threading.Thread(target=job, args=(i, 10, got[i])) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for outs in got:
+        assert len(outs) == 11
+        for W, H in outs[1:]:
+            assert np.array_equal(W, outs[0][0]) and np.array_equal(H, outs[0][1])
+
+
 @pytest.mark.parametrize("iters,log_every", [(7, 0), (5, 2)])
 def test_small_problem_without_room_for_its_launch(torch_cuda, capfd, iters, log_every):
     """Where the runtime refuses the cooperative launch of the small-problem kernel (the process may use
