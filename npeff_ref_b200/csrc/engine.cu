@@ -137,6 +137,7 @@ struct dnpeff_engine {
     float* small_carry = nullptr;
     float* small_partial = nullptr;
     unsigned int* small_barrier = nullptr;
+    bool small_ready = false;     // all of them, with the cuts made
 
     double a_sq = 0.0, a_sum = 0.0;
     double a_sq_global = -1.0;
@@ -358,6 +359,12 @@ void dev_free(dnpeff_engine* e, T*& p) {
     p = nullptr;
 }
 
+void free_small(dnpeff_engine* e) {
+    dev_free(e, e->small_cuts); dev_free(e, e->small_carry);
+    dev_free(e, e->small_partial); dev_free(e, e->small_barrier);
+    e->small_ready = false;
+}
+
 void free_matrix(dnpeff_engine* e) {
     dev_free(e, e->a_vals); dev_free(e, e->a_col); dev_free(e, e->a_rowptr);
     dev_free(e, e->c_vals); dev_free(e, e->c_row); dev_free(e, e->c_colptr);
@@ -373,8 +380,7 @@ void free_matrix(dnpeff_engine* e) {
     dev_free(e, e->gram_scratch);
     dev_free(e, e->tc_scratch);
     e->gram_scratch_floats = 0;
-    dev_free(e, e->small_cuts); dev_free(e, e->small_carry);
-    dev_free(e, e->small_partial); dev_free(e, e->small_barrier);
+    free_small(e);
     dev_free(e, e->plan_csr.long_list);
     dev_free(e, e->plan_csc.long_list);
     e->plan_csr = SpmmPlan();
@@ -1278,7 +1284,8 @@ int run_small(dnpeff_engine* e, int iters, int* made) {
     // words that a launch counts in: barrier, abort flag, chunks of either Gram matrix, then a flag per worker of either side
     const size_t most = (size_t)kNumSMs * small_workers_per_block(ld), sync_words = 4 + 2 * most;
     const int w_workers = small_workers(e->n, e->nnz, ld), h_workers = small_workers(e->ms, e->nnz, ld);
-    if (!e->small_cuts) {
+    if (!e->small_ready) {
+        free_small(e);  // what an earlier call got before memory ran out
         DN_TRY(dev_alloc(e, &e->small_cuts, 2 * (most + 1)));
         DN_TRY(dev_alloc(e, &e->small_carry, 2 * most * ld));
         DN_TRY(dev_alloc(e, &e->small_partial, 2 * partial));
@@ -1290,6 +1297,7 @@ int run_small(dnpeff_engine* e, int iters, int* made) {
                                                                        e->small_cuts + most + 1);
         DN_LAUNCH_CHECK();
         DN_COUNT_LAUNCH(2);
+        e->small_ready = true;
     }
     unsigned int* const words = e->small_barrier;
     SmallArgs a;

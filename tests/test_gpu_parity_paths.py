@@ -499,6 +499,45 @@ def test_small_problem_without_room_for_its_launch(torch_cuda, capfd, iters, log
     assert capfd.readouterr().out.count("step ") == (iters // log_every if log_every else 0)
 
 
+def test_small_problem_after_memory_ran_out(torch_cuda):
+    """A run that finds no memory for the one-launch kernel's buffers says so, and the next one, with memory again,
+    makes them all.  The engine's 64 MB slab is filled to different degrees by H, so that in some of the sizes the partials
+    (19 MB) do not fit behind the smaller buffers, and the device has no room for another slab."""
+    from npeff_ref_b200 import MuNmfParams, DnpeffError, release_memory
+    torch = torch_cuda
+    n, r, failed = 40, 128, 0
+    for m in range(60000, 120001, 10000):
+        rng = np.random.default_rng(m)
+        idx = rng.permutation(m).astype(np.int32).reshape(n, m // n)   # every column once
+        vals = rng.random((n, m // n), dtype=np.float32)
+
+        def engine():
+            eng = _engine(MuNmfParams(rank=r, eps=1e-8, seed=2, init_scale=0.1), keep_memory=False)
+            eng.set_csr(n, m, vals, idx, None, m // n, None, 1)
+            eng.export_shard_csc()                                     # (built in full)
+            eng.init_factors()
+            return eng
+
+        with engine() as eng:
+            eng.run(3, log_every=0)
+            want = eng.load_w_to_host(), eng.load_h_to_host()
+        with engine() as eng:
+            release_memory()
+            torch.cuda.empty_cache()
+            filler = torch.empty(torch.cuda.mem_get_info()[0] - (40 << 20), dtype=torch.uint8, device="cuda")
+            try:
+                eng.run(3, log_every=0)
+            except DnpeffError as e:
+                assert e.code == -2 and "cudaMalloc" in str(e)
+                failed += 1
+            del filler
+            torch.cuda.empty_cache()
+            eng.init_factors()
+            eng.run(3, log_every=0)
+            assert np.array_equal(eng.load_w_to_host(), want[0]) and np.array_equal(eng.load_h_to_host(), want[1])
+    assert failed > 0
+
+
 @pytest.mark.parametrize("keep", [False, True])
 def test_device_memory_after_destroy(torch_cuda, keep):
     """dnpeff_destroy gives the device memory back; with keep_memory it stays for the next engine, which
