@@ -1089,6 +1089,8 @@ int build_csc(dnpeff_engine* e, bool full = false) {
         trace.mark("(before CSC build)");
         const bool tail_only = e->x2 != nullptr && !full;
         const int64_t base = tail_only ? e->hot_nnz : 0;
+        dev_free(e, e->c_vals);  // of a build that failed
+        dev_free(e, e->c_row);
         DN_TRY(dev_alloc(e, &e->c_vals, (size_t)(e->nnz - base)));
         DN_TRY(dev_alloc(e, &e->c_row, (size_t)(e->nnz - base)));
         e->c_base = base;

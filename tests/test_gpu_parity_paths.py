@@ -538,6 +538,24 @@ def test_small_problem_after_memory_ran_out(torch_cuda):
     assert failed > 0
 
 
+def test_failed_csc_builds_hold_no_memory(torch_cuda):
+    """A matrix with a column twice in a row is refused when the CSC is built, and every time anew: the arrays of
+    the builds that failed (80 MB each) do not add up."""
+    from npeff_ref_b200 import MuNmfParams, DnpeffError
+    n, k = 2000, 5000
+    idx = np.tile(np.arange(k, dtype=np.int32), (n, 1))
+    idx[7, 5] = idx[7, 6]
+    vals = np.ones((n, k), np.float32)
+    free = []
+    with _engine(MuNmfParams(rank=20), keep_memory=False) as eng:
+        eng.set_csr(n, k, vals, idx, None, k, None, 1)
+        for _ in range(6):
+            with pytest.raises(DnpeffError, match="twice"):
+                eng.export_shard_csc()
+            free.append(torch_cuda.cuda.mem_get_info()[0])
+    assert free[0] - free[-1] < (100 << 20), free
+
+
 @pytest.mark.parametrize("keep", [False, True])
 def test_device_memory_after_destroy(torch_cuda, keep):
     """dnpeff_destroy gives the device memory back; with keep_memory it stays for the next engine, which
