@@ -497,7 +497,7 @@ __device__ __forceinline__ void small_mma_gx(uint32_t tmem, const float* X, uint
     constexpr int kRows = SmallShape<LD>::kTile;
     const uint32_t idesc = tc_idesc_tf32(128, kRows);
     small_mma_run(tmem + SmallTmem<LD>::kD, tmem + SmallTmem<LD>::kG, LD, X, kRows, 0, 8, idesc);
-    if constexpr (LD > 64) small_mma_run(tmem + SmallTmem<LD>::kD + kRows, tmem + SmallTmem<LD>::kG, LD, X, kRows, 8, LD / 8, idesc);
+    small_mma_run(tmem + SmallTmem<LD>::kD + kRows, tmem + SmallTmem<LD>::kG, LD, X, kRows, 8, LD / 8, idesc);
     tc_commit(bar);
 }
 
@@ -510,7 +510,7 @@ __device__ __forceinline__ void small_update_tc(const SmallArgs& a, const SmallS
     const int w = t >> 5, c = 32 * (w & 3) + (t & 31), j0 = R * (w >> 2);
     const bool mine = 32 * (w & 3) < LD && j0 < tl.rows;  // uniform per warp
     float* const out = s.X + (int64_t)(tl.row0 + j0) * LD + c;
-    float n[R], d[R];
+    float n[R], d[R], e[R];
 #pragma unroll
     for (int j = 0; j < R; j++) x[j] = mine && j0 + j < tl.rows ? __ldcg(out + j * LD) : 0.f;
 #pragma unroll
@@ -519,18 +519,16 @@ __device__ __forceinline__ void small_update_tc(const SmallArgs& a, const SmallS
     mma_wait();
     if (!mine) return;
     const uint32_t at = tmem + SmallTmem<LD>::kD + ((uint32_t)(32 * (w & 3)) << 16) + (uint32_t)j0;
-    if constexpr (R == 16) tc_ld16(at, d);
-    else tc_ld8(at, d);
-    if constexpr (LD > 64) {
-        float e[R];
-        if constexpr (R == 16) tc_ld16(at + S::kTile, e);
-        else tc_ld8(at + S::kTile, e);
-        tc_ld_wait();
-#pragma unroll
-        for (int j = 0; j < R; j++) d[j] += e[j];
+    if constexpr (R == 16) {
+        tc_ld16(at, d);
+        tc_ld16(at + S::kTile, e);
     } else {
-        tc_ld_wait();
+        tc_ld8(at, d);
+        tc_ld8(at + S::kTile, e);
     }
+    tc_ld_wait();
+#pragma unroll
+    for (int j = 0; j < R; j++) d[j] += e[j];
     float q[R], chk = 0.f, r_min = 1.0f;
     uint32_t lowest = 0xffffffffu;
 #pragma unroll
