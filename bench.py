@@ -45,7 +45,7 @@ UNIT = "iter/s"
 
 # dram__bytes_read.sum + dram__bytes_write.sum of one sparse product (a sequence of launches: the dense
 # popular block on tensor cores, then the tail), keyed by (config, ranks, product).  Config 2 on one GPU: both
-# products captured whole at this size (profiles/spmm_products_config2_dram_bytes.md), 17.0 + 0.3 GB and 14.5 + 2.3 GB.
+# products captured whole at this size: 17.0 + 0.3 GB and 14.5 + 2.3 GB.
 NCU_TRAFFIC_BYTES = {(2, 1, "spmm_ah"): 17.34e9, (2, 1, "spmm_wa"): 16.81e9}
 
 

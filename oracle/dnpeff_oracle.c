@@ -12,7 +12,7 @@
  * tree (cc/cuda_lrm_npeff/src/preprocess/column_pruning_test.cc:12-105), whose
  * algorithm is the same scheme as util/sparse_util.h:79-159; this oracle is
  * checked against those four cases.  Where the reference engine could be run
- * on a GPU box from the harness in this folder, its outputs are committed as
+ * (by the harness in this folder, which needs a GPU), its outputs are committed as
  * fixtures and this oracle is checked against them as well.
  *
  * Layouts used here (all fp32 storage):

@@ -171,7 +171,7 @@ def test_op_mu_update_matches_oracle(torch_cuda, rows, r):
 def test_op_mu_update_zero_and_tiny_numerators(torch_cuda, rows, r):
     """Numerators that are exactly zero or below 2^-100, and rows of X that are zero (their
     denominators are then eps alone): the tensor-core update kernels of ranks 64 and 128
-    leave their branch-free division for the IEEE one on such batches; every kernel must
+    do such batches again, tiny numerators scaled (quot_careful); every kernel must
     still give the reference's x * (num / (den + eps))."""
     from npeff_ref_b200._lib import lib, check
     torch = torch_cuda
