@@ -342,7 +342,7 @@ __device__ __forceinline__ void small_add_pieces(F& x, const SmallArgs& a, const
 }
 
 // Few partials (8 at stride 32, 2 at 64): the worker sums all of G for itself.  In a fixed order and in double, as below.  (us an iteration
-// at 8 and 32: 185 x 2695, rank 12, 14.1, 17.2; 64 x 2048, rank 32, 16.4, 18.2; 64 of them 24 and 18.)
+// at 8 and at 32 or 64 allowed: 64 x 2048 x 96 values, rank 32, 16.1, 17.3; 185 x 2695 x 150, rank 12, with 64 of them 16.9, 27.4.)
 template <int LD>
 __device__ __forceinline__ bool small_gram_direct(int partials) { return !SmallShape<LD>::kWide && partials * LD * LD <= 8192; }
 template <int LD>
@@ -971,13 +971,13 @@ inline bool small_rank_ok(int ld) { return ld == 32 || ld == 64 || ld == 96 || l
 
 inline int small_workers_per_block(int ld) { return ld > 64 ? 1 : 2; }
 
-// What updating a row takes, in gathers of a factor row (us per iteration at half, this and 1.5 times this: 2048 x 65536, rank 32,
-// 172, 167, 167; 1738 x 186396 x 3055 values, 32, 159, 154, 161; 300 x 9000 x 1500, 128, 60, 60, 61; 832 x 11990 x 1199, 94, 97, 89, 89).
+// What updating a row takes, in gathers of a factor row (us per iteration at half, this and 1.5 times this: 2048 x 65536 x 4096
+// values, rank 32, 175, 162, 163; 1738 x 186396 x 3055, 32, 168, 152, 154; 300 x 9000 x 1500, 128, 62, 59, 62; 832 x 11990 x 1199, 94, 97, 87, 91).
 inline uint32_t small_row_cost(int ld) { return (uint32_t)(ld <= 64 ? 8 + ld / 2 : 4 + ld / 3); }
 
 // Workers of a side: as many as there are, but each with the work of 600 gathers, or 384 at the wide strides, whose tiles take time by
-// runs of 16 rows (us an iteration at 600 and 1024: 185 x 2695, rank 12, 14.1, 15.5; 969 x 6722, rank 33, 27.2, 29.6; 64 x 2048, rank 32,
-// 16.4, 15.8, and 20 or more from 1500 on; 458 x 2551, rank 96: 32 at 384, 36 at 1024).
+// runs of 16 rows (us an iteration at these and at 1024: 185 x 2695 x 150 values, rank 12, 16.9, 17.3; 64 x 2048 x 96, rank 32,
+// 16.1, 15.6, and 20 or more from 1500 on; 400 x 8000 x 300, 32, 969 x 6722 x 400, 33, and 458 x 2551 x 300, 96, even).
 inline int small_workers(int64_t rows, int64_t entries, int ld) {
     const int64_t cost = entries + rows * small_row_cost(ld);
     const int64_t most = (int64_t)kNumSMs * small_workers_per_block(ld);
@@ -987,17 +987,17 @@ inline int small_workers(int64_t rows, int64_t entries, int ld) {
 // Whether these launches beat the large path.  An iteration takes about 15 us, two gathers of a factor row per stored entry, and the two
 // contractions.  The large path takes 65 to 105 us plus the same gathers, but does the popular columns densely and contracts at the
 // tensor cores' full rate.  us an iteration here and there:
-//   stride 32: 8000 x 600000 x 4000 values 694, 795; 500 x 600000 x 20000 341, 501; 17000 x 200000 x 1800 525, 570; 3000 x 60000 x 4000
-//              213, 237; 20000 x 50000 x 1500 477, 454; 5000 x 20000 x 3000 239, 221
-//   64: 2000 x 40000 x 2000 168, 171; 1000 x 200000 x 2000 221, 227; 5000 x 50000 x 1000 203, 191; 3001 x 100003 x 2047 312, 250
-//   96: 12000 x 12000 x 150 142, 165; 200 x 100000 x 3000 144, 169; 3060 x 80340 x 368 176, 170; 1500 x 60000 x 1500 217, 205
-//   128: 800 x 40000 x 1000 118, 172; 200 x 100000 x 3000 159, 181; 4000 x 40000 x 300 160, 160; 828 x 74164 x 8240 560, 284
+//   stride 32: 8000 x 600000 x 4000 values 702, 763; 500 x 600000 x 20000 355, 468; 17000 x 200000 x 1800 560, 571; 3000 x 60000 x 4000
+//              214, 237; 20000 x 50000 x 1500 507, 454; 5000 x 20000 x 3000 245, 227
+//   64: 2000 x 40000 x 2000 165, 171; 1000 x 200000 x 2000 221, 228; 5000 x 50000 x 1000 204, 195; 3001 x 100003 x 2047 280, 250
+//   96: 12000 x 12000 x 150 140, 165; 200 x 100000 x 3000 146, 170; 3060 x 80340 x 368 163, 170; 1500 x 60000 x 1500 215, 208
+//   128: 800 x 40000 x 1000 118, 173; 200 x 100000 x 3000 161, 185; 4000 x 40000 x 300 144, 162; 828 x 74164 x 8240 523, 289
 // popular: stored entries in popular columns; block: elements of the dense block.
 inline bool small_pays(int64_t nnz, int64_t rows, int ld, int64_t popular, int64_t block) {
     if (ld == 32) {
         // Here large problems can gain too, and what decides is how dense the popular columns are.  us per million gathers, per MB of
-        // the dense block and per MB of factors and numerators, from fourteen shapes (here within 3 %, there 8, but for the least): the
-        // large path where the two are about even.
+        // the dense block and per MB of factors and numerators, from fourteen shapes (here within 3 % with the 1.04 below, there 8, but
+        // for the least): the large path where the two are about even.
         const double gathers = 2e-6 * (double)nnz, factors = 384e-6 * (double)rows;
         const double here = 7.5 * gathers + 0.84 * factors;
         const double there = 73.0 + 6.8 * 2e-6 * (double)(nnz - popular) + 0.18 * 8e-6 * (double)block + 1.47 * factors;
