@@ -111,7 +111,7 @@ int dnpeff_release_memory(int device);
  *   "keep_memory"       1: dnpeff_destroy leaves the engine's device memory, up to 8 GB a
  *                       device with what lies there already, for the next engine of
  *                       the process: for programs that run one job after the other
- *                       (allocating and freeing is a quarter of a small one's time).  It
+ *                       (allocating and freeing is a sixth of a small one's time).  It
  *                       goes back to the device when an allocation of this library
  *                       fails, when an engine with this option ends that never needed
  *                       it, and with dnpeff_release_memory; no other allocator can

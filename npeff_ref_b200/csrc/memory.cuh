@@ -12,7 +12,7 @@ namespace dnpeff {
 
 // Slabs that engines left when they were destroyed (those that were asked to, option keep_memory), for
 // the next engine on the same device: whole jobs from host memory, 300 x 9000 at rank 128 and 8192 x 1048576
-// at rank 64 (4 GB of slabs each), take 6.8 and 77 ms without and 5.1 and 63 with it, the
+// at rank 64 (4 GB of slabs each), take 5.1 and 77 ms without and 4.2 and 62 with it, the
 // rest being cudaMalloc and cudaFree.  At most kMost bytes a device, a twentieth of its memory; they go back to the
 // device when an allocation here fails, when an engine ends that never needed them, and with dnpeff_release_memory.
 class SlabCache {
