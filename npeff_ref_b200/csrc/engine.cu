@@ -1052,11 +1052,12 @@ int fill_csc(dnpeff_engine* e, int mode) {
     }
     // a column longer than kCscShortMax needs that many rows; how many there are stays on the device
     if (e->n > kCscShortMax) {
-        if (bitmap_bytes > 200 * 1024) {
+        if (e->n > kCscLongRows) {
             int h_long = 0;
             DN_TRY(read_small(e, n_long.p, sizeof(int), &h_long));
             if (h_long > 0)
-                return fail(DNPEFF_ERR_UNSUPPORTED, "columns longer than 512 entries need n_rows <= 819200");
+                return fail(DNPEFF_ERR_UNSUPPORTED, "columns longer than %d entries need n_rows <= %lld", kCscShortMax,
+                            (long long)kCscLongRows);
         } else {
             DN_CUDA(cudaFuncSetAttribute(k_csc_order_long, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bitmap_bytes));
             const int64_t blocks = std::min<int64_t>(col_last - col_first, (int64_t)kNumSMs * 8);
@@ -1274,6 +1275,8 @@ int step_h(dnpeff_engine* e) {
 bool small_problem(const dnpeff_engine* e) {
     if (!tensor_cores_enabled() || e->timing || e->p.n_shards > 1 || !small_rank_ok(e->ld)) return false;
     if (e->n <= 0 || e->ms <= 0 || e->nnz <= 0 || e->nnz > ((int64_t)1 << 30)) return false;
+    // the large path leaves the popular columns out of its CSC, where they could not be put in order
+    if (e->n > kCscLongRows && e->n_hot > 0) return false;
     return small_pays(e->nnz, e->n + e->ms, e->ld, e->hot_nnz, e->n * e->n_hot);
 }
 

@@ -297,6 +297,7 @@ __global__ void k_csc_scatter(const int64_t* __restrict__ rowptr, const int32_t*
 }
 
 constexpr int kCscShortMax = 512;  // longest column ranked by comparison (keys per warp in shared memory)
+constexpr int64_t kCscLongRows = 819200;  // rows up to which longer columns can be ordered: their bitmap and its sums take 200 KB
 
 // Columns [col_first, col_last) with at most kCscShortMax entries: one warp per column.  The row order is that of the set bits in a
 // bitmap of the rows where they fit the warp's shared memory and the column is long against it, else by comparing every pair.  The

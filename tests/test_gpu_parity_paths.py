@@ -472,6 +472,40 @@ def test_small_problems_of_two_engines_at_once(torch_cuda):
             assert np.array_equal(W, outs[0][0]) and np.array_equal(H, outs[0][1])
 
 
+@pytest.mark.parametrize("popular", [8, 0])
+def test_small_problem_with_more_rows_than_a_long_column_can_have(torch_cuda, popular):
+    """Rank 32 with 820 000 rows of two entries, just past the rows up to which a column of more than 512 entries can be put in row
+    order: with popular columns (102 500 entries each) the one-launch kernel, which needs them in the CSC, would be refused what
+    the large path does; without them it runs.  Against the oracle and single steps, and by the number of launches."""
+    from npeff_ref_b200 import MuNmfParams
+    rng = np.random.default_rng(popular)
+    n, m, r, iters, eps = 820000, 4000, 32, 2, 1e-8
+    rows = np.arange(n)
+    ind = np.stack([rng.permutation(rows) % (popular or m // 2), m // 2 + rng.permutation(rows) % (m // 2)], axis=1).astype(np.int32)
+    vals = rng.random((n, 2), dtype=np.float32) + np.float32(0.1)
+    with _engine(MuNmfParams(rank=r, eps=eps, seed=6, init_scale=0.3)) as eng:
+        eng.set_csr(n, m, vals, ind, None, 2, None, 1)
+        mk = eng.shape[1]
+        assert eng.layout()[0] == popular
+        W0, H0 = O.init_factors(n, mk, r, 6, 0.3)
+        for _ in range(2):
+            eng.init_factors()
+            launches = eng.launch_count()
+            eng.run(iters, log_every=0)
+            launches = eng.launch_count() - launches
+        assert (launches == 1) == (popular == 0)
+        got = eng.load_w_to_host(), eng.load_h_to_host()
+        eng.init_factors()
+        for _ in range(iters):
+            eng.step_w()
+            eng.step_h()
+        steps = eng.load_w_to_host(), eng.load_h_to_host()
+    v, c, rp, n2o = O.prune_columns(vals.ravel(), ind.ravel(), np.arange(0, 2 * n + 1, 2, dtype=np.int64), m, 1)
+    want = O.run(v, c, rp, mk, W0, H0, iters, eps, acc64=True, losses=True)
+    for g, s, o in zip(got, steps, want):
+        assert rel_fro(g, o) < 1e-5 and rel_fro(g, s) < 1e-5
+
+
 @pytest.mark.parametrize("iters,log_every", [(7, 0), (5, 2)])
 def test_small_problem_without_room_for_its_launch(torch_cuda, capfd, iters, log_every):
     """Where the runtime refuses the cooperative launch of the small-problem kernel (the process may use
