@@ -319,8 +319,11 @@ def test_small_problems_in_one_launch(torch_cuda, n, m, lens, r):
         W0, H0 = O.init_factors(n, mk, r, 6, 0.3)
         for _ in range(2):
             eng.init_factors()
+            launches = eng.launch_count()
             eng.run(iters, log_every=0)
+            launches = eng.launch_count() - launches
             got.append((eng.load_w_to_host(), eng.load_h_to_host()))
+        assert launches == 1  # (the first run makes the CSC as well)
         eng.init_factors()
         for _ in range(iters):
             eng.step_w()
@@ -336,7 +339,8 @@ def test_small_problems_in_one_launch(torch_cuda, n, m, lens, r):
 @pytest.mark.parametrize("n,m,lens,r", [
     (65, 3000, (40, 41), 96), (129, 2600, (1, 60), 128),      # a row more than a tile, or a half, of the wide strides
     (600, 900, (300, 301), 100), (2400, 70, (30, 60), 96),    # rows cut over many workers; more rows than tiles on W's side
-    (40, 50000, (2000, 2100), 64), (16, 20000, (6000, 6001), 128)])  # several tiles a worker on H's
+    (40, 50000, (2000, 2100), 64), (16, 20000, (6000, 6001), 128),   # several tiles a worker on H's
+    (24, 20000, (3000, 3001), 96), (24, 26000, (3000, 3001), 90)])
 def test_small_problem_tiles_and_tiny_values(torch_cuda, n, m, lens, r):
     """The one-launch kernel around its tiles and cuts, and with components so small that numerators fall below 2^-100
     and below the normal range: against single steps and the oracle."""
@@ -350,8 +354,12 @@ def test_small_problem_tiles_and_tiny_values(torch_cuda, n, m, lens, r):
         W0, H0 = O.init_factors(n, mk, r, 6, 0.3)
         H0[::5] *= np.float32(1e-33)
         H0[1::7] *= np.float32(1e-38)
-        eng.init_factors(W0, H0)
-        eng.run(iters, log_every=0)
+        for _ in range(2):
+            eng.init_factors(W0, H0)
+            launches = eng.launch_count()
+            eng.run(iters, log_every=0)
+            launches = eng.launch_count() - launches
+        assert launches == 1  # (the first run makes the CSC as well)
         got = eng.load_w_to_host(), eng.load_h_to_host()
         eng.init_factors(W0, H0)
         for _ in range(iters):
